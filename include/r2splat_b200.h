@@ -376,6 +376,23 @@ int r2s_raster_record_bwd(int dtype, const void* records, const uint16_t* rects,
                           uint32_t C, uint32_t N, uint32_t width, uint32_t height, uint32_t tile_size,
                           void* grads, void* v_means2d_abs, void* v_uncertainties, void* stream);
 
+/* Tile-parallel VJP of r2s_raster_render for fp32 Gaussian records with the
+ * variance branch (v_render_var and v_uncertainties non-null), over the sorted
+ * lists (tile sizes 8, 16 and 32, image sides below 65536): each (tile, record)
+ * pair writes its sums to a slot of its own (slots: slot_capacity x 8
+ * floats), numbered by tile_cum, the inclusive scan of the records' tile counts
+ * over [C,N], and a second pass adds each record's slots in order into grads
+ * [C,N,8] (every record written; no atomics). Same adjoints, decisions and null
+ * conventions as r2s_raster_record_bwd. n_used: the intersection count kept on
+ * the device (capacity-bounded steps), or null; slots past slot_capacity are
+ * neither written nor read. records, slots and grads must be 32-byte aligned. */
+int r2s_raster_tile_bwd(const float* records, const uint16_t* rects, const float* uncertainties,
+                        int detach_variance, const int32_t* tile_offsets, const int32_t* flatten_ids,
+                        uint64_t n_isects, const int64_t* n_used, const int64_t* tile_cum, const float* v_render,
+                        const float* v_render_var, uint32_t C, uint32_t N, uint32_t width, uint32_t height,
+                        uint32_t tile_size, uint32_t tiles_x, uint32_t tiles_y, float* slots,
+                        uint64_t slot_capacity, float* grads, float* v_uncertainties, void* stream);
+
 /* out [N] = sum over cameras c of per_record [C,N], in camera order (the
  * record VJP's uncertainty adjoints; no reference counterpart as a call: the
  * reference adds them with atomics inside K20/K22). */

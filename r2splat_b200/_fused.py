@@ -6,9 +6,11 @@ Rasterize (the reference's explicit.py:160-183 and :204-241):
   read of the intersection count -> emission + stable radix sort + per-tile
   offsets -> tile accumulation. The VJP needs no tile order: one warp per
   (camera, primitive) record walks the pixels of the record's tile rectangle
-  and writes its packed adjoints [C,N,8] once, then one per-primitive
-  chain-rule pass (conic/mu VJP, projection VJP summed over cameras, Beta path
-  factor, parameter-transform VJP); neither uses atomics.
+  and writes its packed adjoints [C,N,8] once; that of fp32 Gaussians with the
+  variance branch is tile-parallel over the sorted lists, one slot per (tile,
+  record) pair, summed per record in a fixed order. Then one per-primitive chain-rule pass (conic/mu VJP,
+  projection VJP summed over cameras, Beta path factor, parameter-transform
+  VJP). No atomics.
 
 Voxelize (explicit.py:286-307, :331-350): the same structure in 3D with
 64-byte records [N,16]. Its VJP is tile-parallel over the sorted lists, but
@@ -37,6 +39,10 @@ from .cuda import _wrapper as low
 Tensor = torch.Tensor
 RASTER_TILE = 16
 VOXEL_TILE = 8
+# Largest scratch the tile-parallel raster VJP takes for its per-intersection slots (32 bytes each); past it
+# the VJP walks the records' tile rectangles instead.
+RASTER_SLOT_BUDGET_BYTES = 8 << 30
+RASTER_SLOT_BYTES = 32
 # Largest scratch the deterministic voxel VJP takes for its per-intersection slots (12 values each);
 # past it the VJP walks the primitives' tile boxes instead (one slot per primitive and z-layer).
 VOXEL_SLOT_BUDGET_BYTES = 8 << 30
@@ -149,35 +155,72 @@ def raster_intersections(means, covars, densities, beta, ratio, viewmats, Ks, wi
                          tile_size=RASTER_TILE, before_count=None):
     """Projection + packing + sorted tile intersections.
 
-    Returns (records, offsets, isect_ids, flatten_ids, M, rects); rects [C,N,4] are the tile rectangles.
+    Returns (records, offsets, isect_ids, flatten_ids, M, rects, cum); rects [C,N,4] are the tile rectangles and
+    cum the inclusive scan of the per-record tile counts, which the VJP's slots are numbered by.
     ``before_count`` runs just before the host reads the intersection count (the pending input checks).
     """
+    records, rects, counts = _raster_project(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps,
+                                             radius_clip, tile_size)
+    cum = _raster_scan(counts)
+    if before_count is not None:
+        before_count()
+    m = int(cum[-1].item())
+    isect_ids, flatten_ids, offsets = _raster_lists(rects, cum, m, width, height, tile_size)
+    return records, offsets, isect_ids, flatten_ids, m, rects, cum
+
+
+def _raster_project(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps, radius_clip, tile_size):
+    """Records [C,N,8], tile rectangles [C,N,4] and tile counts [C,N]."""
     device = means.device
     c, n = viewmats.shape[0], means.shape[0]
     tx = (width + tile_size - 1) // tile_size
     ty = (height + tile_size - 1) // tile_size
-    stream = _stream(device)
-    lib = _backend.library()
     records = means.new_empty((c, n, 8))
     rects = torch.empty((c, n, 4), dtype=torch.int16, device=device)
     counts = torch.empty((c, n), dtype=torch.int32, device=device)
     _backend.call("r2s_raster_project", _dtype(means), _ptr(means), _ptr(covars), _ptr(densities), _ptr(beta),
                   _ptr(ratio), _ptr(viewmats), _ptr(Ks), c, n, width, height, float(eps), float(eps),
-                  float(radius_clip), tile_size, tx, ty, _ptr(records), _ptr(rects), _ptr(counts), stream)
-    cum = torch.empty((c * n,), dtype=torch.int64, device=device)
-    ws = _ws(lib.r2s_isect_count_workspace(c * n), device)
-    _backend.call("r2s_scan_tile_counts", _ptr(counts), c * n, _ptr(cum), _ptr(ws), ws.numel(), stream)
-    if before_count is not None:
-        before_count()
-    m = int(cum[-1].item())
+                  float(radius_clip), tile_size, tx, ty, _ptr(records), _ptr(rects), _ptr(counts), _stream(device))
+    return records, rects, counts
+
+
+def _raster_scan(counts):
+    """Inclusive scan [C * N] of the records' tile counts."""
+    cum = torch.empty((counts.numel(),), dtype=torch.int64, device=counts.device)
+    ws = _ws(_backend.library().r2s_isect_count_workspace(counts.numel()), counts.device)
+    _backend.call("r2s_scan_tile_counts", _ptr(counts), counts.numel(), _ptr(cum), _ptr(ws), ws.numel(),
+                  _stream(counts.device))
+    return cum
+
+
+def _raster_lists(rects, cum, m, width, height, tile_size):
+    """Sorted tile lists (isect_ids, flatten_ids, offsets) of the m intersections of tile rectangles."""
+    device = rects.device
+    c, n = rects.shape[:2]
+    tx = (width + tile_size - 1) // tile_size
+    ty = (height + tile_size - 1) // tile_size
     isect_ids = torch.empty((m,), dtype=torch.int64, device=device)
     flatten_ids = torch.empty((m,), dtype=torch.int32, device=device)
     offsets = torch.empty((c, ty, tx), dtype=torch.int32, device=device)
-    ws = _ws(lib.r2s_isect_emit_workspace(m, c * tx * ty), device)
+    ws = _ws(_backend.library().r2s_isect_emit_workspace(m, c * tx * ty), device)
     with _stage("raster_sort"):
         _backend.call("r2s_raster_emit", _ptr(rects), c, n, tx, ty, _ptr(cum), m, _ptr(isect_ids),
-                      _ptr(flatten_ids), _ptr(offsets), _ptr(ws), ws.numel(), stream)
-    return records, offsets, isect_ids, flatten_ids, m, rects
+                      _ptr(flatten_ids), _ptr(offsets), _ptr(ws), ws.numel(), _stream(device))
+    return isect_ids, flatten_ids, offsets
+
+
+def raster_vjp_takes_tiles(dtype, beta: bool, variance: bool, tile_size, width, height, n_slots) -> bool:
+    """Whether the raster VJP runs tile-parallel over the lists (r2s_raster_tile_bwd) rather than record by record.
+
+    fp32 Gaussians with a variance adjoint, on tile sizes of whole 8x8 blocks: the tile walk evaluates whole blocks,
+    which pays for Gaussian boxes (317 pixels on average in the cone-beam scene; 1.06 -> 0.57 ms at 50,021 primitives
+    and 17 views of 333 x 517) and not for the compact Beta records (42 pixels; 0.31 ms by records, 0.46 ms by tiles
+    at 100,000 primitives and 32 views of 384^2). Without a variance adjoint the record walk keeps the sums' order.
+    The rule depends on the scene alone, not on whether the lists are still held, so a rebuilt backward gives the same
+    gradients.
+    """
+    return (variance and dtype == torch.float32 and not beta and tile_size in (8, 16, 32)
+            and max(width, height) < 65536 and n_slots * RASTER_SLOT_BYTES <= RASTER_SLOT_BUDGET_BYTES)
 
 
 IMAGE_LOSS_KINDS = {"mse": 0, "l1": 1}  # R2S_IMAGE_LOSS_MSE, R2S_IMAGE_LOSS_L1
@@ -216,7 +259,7 @@ def raster_forward(means, quats, scales, densities, viewmats, Ks, width, height,
     c = viewmats.shape[0]
     covars, _ = low.parameter_transform_fwd(quats, scales)
     ratio = _beta.beta_path_ratio(beta) if beta is not None else None
-    records, offsets, isect_ids, flatten_ids, m, rects = raster_intersections(
+    records, offsets, isect_ids, flatten_ids, m, rects, cum = raster_intersections(
         means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps, radius_clip, tile_size,
         before_count)
     image = means.new_empty((c, height, width))
@@ -235,7 +278,7 @@ def raster_forward(means, quats, scales, densities, viewmats, Ks, width, height,
                                          means.shape[0], width, height, tile_size, target, kind, weight, image,
                                          variance, device)
     state = RasterState(covars, records, offsets, isect_ids, flatten_ids, ratio, m, width, height, tile_size,
-                        extra={"rects": rects})
+                        extra={"rects": rects, "cum": cum})
     output = image if uncertainty is None else (image, variance)
     if image_loss is None:
         return output, state
@@ -243,25 +286,18 @@ def raster_forward(means, quats, scales, densities, viewmats, Ks, width, height,
 
 
 def raster_vjp_state(means, quats, scales, densities, viewmats, Ks, width, height, beta, eps, radius_clip,
-                     tile_size=RASTER_TILE):
+                     tile_size=RASTER_TILE, n_isects=0):
     """What the raster VJP reads (covariances, packed records, tile rectangles), rebuilt without the image.
 
-    The record-parallel VJP needs neither the intersection lists nor their
-    order, so recomputation is the parameter transform and the projection only.
+    ``n_isects`` is the forward's intersection count of the same inputs; the VJP rebuilds the tile lists from it where
+    it reads them.
     """
-    device = means.device
-    c, n = viewmats.shape[0], means.shape[0]
-    tx = (width + tile_size - 1) // tile_size
-    ty = (height + tile_size - 1) // tile_size
     covars, _ = low.parameter_transform_fwd(quats, scales)
     ratio = _beta.beta_path_ratio(beta) if beta is not None else None
-    records = means.new_empty((c, n, 8))
-    rects = torch.empty((c, n, 4), dtype=torch.int16, device=device)
-    counts = torch.empty((c, n), dtype=torch.int32, device=device)
-    _backend.call("r2s_raster_project", _dtype(means), _ptr(means), _ptr(covars), _ptr(densities), _ptr(beta),
-                  _ptr(ratio), _ptr(viewmats), _ptr(Ks), c, n, width, height, float(eps), float(eps),
-                  float(radius_clip), tile_size, tx, ty, _ptr(records), _ptr(rects), _ptr(counts), _stream(device))
-    return RasterState(covars, records, None, None, None, ratio, 0, width, height, tile_size, extra={"rects": rects})
+    records, rects, counts = _raster_project(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps,
+                                             radius_clip, tile_size)
+    return RasterState(covars, records, None, None, None, ratio, n_isects, width, height, tile_size,
+                       extra={"rects": rects, "counts": counts})
 
 
 def voxel_vjp_state(means, quats, scales, densities, shape, extent, center, beta, uncertainty, eps, radius_clip,
@@ -284,15 +320,32 @@ def raster_backward(state: RasterState, means, quats, scales, densities, beta, u
     c, n = viewmats.shape[0], means.shape[0]
     tile = state.tile_size
     stream = _stream(device)
-    grads = means.new_empty((c, n, 8))  # every record is written by the record-parallel VJP
+    grads = means.new_empty((c, n, 8))  # every record is written
     # With the variance branch: one uncertainty adjoint per record, summed over cameras in order.
     v_unc_cn = means.new_empty((c, n)) if v_variance is not None else None
     v_unc = means.new_empty((n,)) if v_variance is not None else None
-    with _stage("raster_render_bwd"):
-        _backend.call("r2s_raster_record_bwd", _dtype(means), _ptr(state.records), _ptr(state.extra["rects"]),
-                      _ptr(uncertainty), int(beta is not None), int(bool(detach_variance)), _ptr(v_image),
-                      _ptr(v_variance), c, n, state.width, state.height, tile, _ptr(grads), None, _ptr(v_unc_cn),
-                      stream)
+    rects, m = state.extra["rects"], state.n_isects
+    if raster_vjp_takes_tiles(means.dtype, beta is not None, v_variance is not None, tile, state.width, state.height,
+                              m):
+        if "cum" not in state.extra:
+            state.extra["cum"] = _raster_scan(state.extra["counts"])
+        if state.offsets is None:
+            _, flatten_ids, offsets = _raster_lists(rects, state.extra["cum"], m, state.width, state.height, tile)
+        else:
+            flatten_ids, offsets = state.flatten_ids, state.offsets
+        with _stage("raster_render_bwd"):
+            slots = means.new_empty((max(m, 1), RASTER_SLOT_BYTES // 4))
+            _backend.call("r2s_raster_tile_bwd", _ptr(state.records), _ptr(rects), _ptr(uncertainty),
+                          int(bool(detach_variance)), _ptr(offsets), _ptr(flatten_ids), m, None,
+                          _ptr(state.extra["cum"]), _ptr(v_image), _ptr(v_variance), c, n, state.width, state.height,
+                          tile, offsets.shape[2], offsets.shape[1], _ptr(slots), slots.shape[0], _ptr(grads),
+                          _ptr(v_unc_cn), stream)
+    else:
+        with _stage("raster_render_bwd"):
+            _backend.call("r2s_raster_record_bwd", _dtype(means), _ptr(state.records), _ptr(rects),
+                          _ptr(uncertainty), int(beta is not None), int(bool(detach_variance)), _ptr(v_image),
+                          _ptr(v_variance), c, n, state.width, state.height, tile, _ptr(grads), None, _ptr(v_unc_cn),
+                          stream)
     if v_unc is not None:
         _backend.call("r2s_sum_over_cameras", _dtype(means), _ptr(v_unc_cn), c, n, _ptr(v_unc), stream)
     log_grad = _beta.beta_path_log_grad(beta) if beta is not None else None
@@ -382,9 +435,9 @@ def voxel_intersections(means, covars, densities, beta, uncertainty, extent, cen
 
 
 def release_lists(state):
-    """Drops a forward state's intersection lists (raster or voxel): neither VJP needs them (the raster VJP
-    walks tile rectangles; the voxel VJP then takes its list-free form), so a caller short of memory can
-    free them between forward and backward. Returns the tensors dropped."""
+    """Drops a forward state's intersection lists (raster or voxel), so a caller short of memory can free them
+    between forward and backward: the raster VJP rebuilds them where it needs them, the voxel VJP then takes its
+    list-free form. Returns the tensors dropped."""
     dropped = [t for t in (state.isect_ids, state.flatten_ids, state.offsets, getattr(state, "packed", None))
                if t is not None]
     state.isect_ids = state.flatten_ids = state.offsets = None

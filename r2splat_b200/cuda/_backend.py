@@ -79,6 +79,10 @@ SIGNATURES: dict[str, tuple] = {
     "r2s_raster_render_bwd": (I32, [I32, P, P, I32, I32, P, P, P, P, U32, U32, U32, U32, U32, U32, U32, U32,
                                     P, P, P, P]),
     "r2s_raster_record_bwd": (I32, [I32, P, P, P, I32, I32, P, P, U32, U32, U32, U32, U32, P, P, P, P]),
+    # records, rects, unc, detach, offsets, ids, n_isects, n_used, tile_cum, v_render, v_render_var, C, N, W, H,
+    # tile, tiles_x, tiles_y, slots, slot_capacity, grads, v_unc, stream
+    "r2s_raster_tile_bwd": (I32, [P, P, P, I32, P, P, U64, P, P, P, P, U32, U32, U32, U32, U32, U32, U32, P, U64, P,
+                                  P, P]),
     "r2s_sum_over_cameras": (I32, [I32, P, U32, U32, P, P]),
     "r2s_raster_chain_bwd": (I32, [I32, P, P, P, P, P, P, P, P, P, U32, U32, U32, U32, F32, F64, P, P, P, P,
                                    P, P, P]),

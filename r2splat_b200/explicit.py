@@ -144,10 +144,10 @@ def release_intersection_lists(context) -> None:
 
     Not part of the reference's surface: a memory-bounded caller (the serving
     loop's recompute-in-backward mode) calls it between ``rasterize_fwd`` /
-    ``voxelize_fwd`` and the matching backward. Neither VJP reads the lists:
-    the raster VJP walks each record's tile rectangle and the voxel VJP then
-    walks each primitive's tile box. The gradients are unchanged up to the
-    voxel VJP's summation order.
+    ``voxelize_fwd`` and the matching backward. The raster VJP rebuilds the
+    lists where it reads them (or walks each record's tile rectangle) and the
+    voxel VJP then walks each primitive's tile box. The gradients are unchanged
+    up to the voxel VJP's summation order.
     """
     if not isinstance(context, _Context) or context.used:
         raise RuntimeError("expected an unconsumed explicit context")
