@@ -414,6 +414,245 @@ __global__ void __launch_bounds__(kMaxThreads) raster_fwd_pair_kernel(
     }
 }
 
+// Forward in fp32 with a hit list per group of lanes, for tile sizes 8, 16 and
+// 32. A group of 2 kBlock lanes owns one kBlock x kBlock pixel block, each lane
+// kBlock / 2 pixels of one column (rows y, y + 2, ...), which share the record's
+// terms in dx and its reads; a warp's groups own neighbouring blocks and walk
+// their lists side by side, padded with a record that contributes nothing.
+// 4x4 blocks evaluate fewer samples than the 8x8 blocks of a whole warp in
+// raster_fwd_pair_kernel: 417 against 565 a record in the cone-beam scene
+// (200,000 Gaussians, 64 views of 512^2), 98 against 192 for compact Beta
+// records (500,000 at 768^2, boxes with a median of 42 pixels). A batch takes
+// one block barrier.
+//
+// The staged record is rewritten in place to what the samples use: a Gaussian's
+// conic diagonal is halved (exact, so sigma needs no separate factor 1/2), o mu
+// is formed once, and the uncertainty takes the last slot. Expressions and list
+// order are raster_fwd_pair_kernel's, so the images are the same bit for bit.
+// A bounded record (see clip_to_record) cannot have a sample with sigma < 0
+// (d^2 < 0) by its box's error bound; a batch that holds any other record takes
+// the strict walk, which tests it.
+//
+// The grid runs over all cameras' tiles row by row, from the middle rows
+// outwards: detectors are centred on the object, so the longest lists start
+// first and the last CTAs are short (with 8x8 blocks at 64 views: 3.86 ms
+// camera by camera, 3.58 ms this way).
+//
+// Measured against the pair kernel (B200): the cone-beam scene 4.30 -> 3.49 ms,
+// one view of 100,000 at 512^2 0.119 -> 0.097 ms, 500,000 Beta records with
+// uncertainty, 128 views of 768^2 10.84 -> 8.03 ms. It is bound by instruction
+// issue (86 % of the slots, Beta; special-function unit 57 %).
+template <bool kBeta, bool kVar, bool kStrict, int kP>
+__device__ __forceinline__ void group_record(const char* rec, float px, const float2 (&py)[kP], float2 (&acc)[kP],
+                                             float2 (&accv)[kP]) {
+    const float4 f0 = *reinterpret_cast<const float4*>(rec);       // x, y (Beta) or -y, a / 2 or a, b
+    const float4 f1 = *reinterpret_cast<const float4*>(rec + 16);  // c / 2 or c, o mu, beta, q
+    if constexpr (!kBeta) {
+        const float dx = px - f0.x;
+        const float2 adx = splat2(__fmul_rn(f0.z, dx)), bdx = splat2(__fmul_rn(f0.w, dx));
+#pragma unroll
+        for (int k = 0; k < kP; ++k) {
+            const float2 dy = add2(py[k], splat2(f0.y));
+            const float2 sigma = fma2(bdx, dy, fma2(adx, splat2(dx), mul2(mul2(splat2(f1.x), dy), dy)));
+            const float2 alpha = mul2(splat2(f1.y), make_float2(exp(-sigma.x), exp(-sigma.y)));
+            if (!((kStrict && sigma.x < 0.f) || fabs(alpha.x) < 1e-5f)) {
+                acc[k].x += alpha.x;
+                if (kVar) accv[k].x = __fmaf_rn(__fmul_rn(f1.w, alpha.x), alpha.x, accv[k].x);
+            }
+            if (!((kStrict && sigma.y < 0.f) || fabs(alpha.y) < 1e-5f)) {
+                acc[k].y += alpha.y;
+                if (kVar) accv[k].y = __fmaf_rn(__fmul_rn(f1.w, alpha.y), alpha.y, accv[k].y);
+            }
+        }
+    } else {
+        const float dx = f0.x - px;
+        const float2 adx = splat2(__fmul_rn(f0.z, dx)), b2dx = splat2(__fmul_rn(__fmul_rn(2.f, f0.w), dx));
+#pragma unroll
+        for (int k = 0; k < kP; ++k) {
+            const float2 dy = add2(splat2(f0.y), make_float2(-py[k].x, -py[k].y));
+            const float2 d2 = fma2(mul2(splat2(f1.x), dy), dy, fma2(adx, splat2(dx), mul2(b2dx, dy)));
+            const bool s0 = !((kStrict && d2.x < 0.f) || d2.x >= 1.f), s1 = !((kStrict && d2.y < 0.f) || d2.y >= 1.f);
+            const float2 h = add2(splat2(1.f), make_float2(-d2.x, -d2.y));
+            const float a0 = s0 ? f1.y * pow(h.x, f1.z) : 0.f;
+            const float a1 = s1 ? f1.y * pow(h.y, f1.z) : 0.f;
+            if (s0 && !(fabs(a0) < 1e-5f)) {
+                acc[k].x += a0;
+                if (kVar) accv[k].x = __fmaf_rn(__fmul_rn(f1.w, a0), a0, accv[k].x);
+            }
+            if (s1 && !(fabs(a1) < 1e-5f)) {
+                acc[k].y += a1;
+                if (kVar) accv[k].y = __fmaf_rn(__fmul_rn(f1.w, a1), a1, accv[k].y);
+            }
+        }
+    }
+}
+
+template <bool kBeta, bool kVar, uint32_t kT, uint32_t kBlock>
+__global__ void __launch_bounds__(2 * kT * kT / kBlock) raster_fwd_group_kernel(
+    const Rec2D<float>* __restrict__ records, const float* __restrict__ uncertainties, uint32_t N,
+    const int32_t* __restrict__ offsets, const int32_t* __restrict__ flatten_ids, int32_t n_isects,
+    const int64_t* __restrict__ n_dev, uint32_t C, uint32_t width, uint32_t height, uint32_t tiles_x,
+    uint32_t tiles_y, float* __restrict__ render, float* __restrict__ render_var, uint32_t B,
+    ImageLossEpilogue<float> loss) {
+    constexpr uint32_t kGroup = 2u * kBlock;            // lanes
+    constexpr uint32_t kLists = 32u / kGroup;           // groups of a warp
+    constexpr uint32_t kBlocks = kT / kBlock;           // blocks along a tile's side
+    constexpr uint32_t kThreads = kBlocks * kBlocks * kGroup;
+    constexpr uint32_t kAcross = 2u, kDown = kLists / 2u;  // a warp's blocks
+    constexpr int kP = int(kBlock) / 4;                 // pixel pairs a lane
+    static_assert(kBlocks * kBlocks <= 32u, "a word of block hits");
+    extern __shared__ __align__(16) unsigned char smem[];
+    Rec2D<float>* s_rec = reinterpret_cast<Rec2D<float>*>(smem);          // [3][B + 1], the last one empty
+    uint32_t* s_hit = reinterpret_cast<uint32_t*>(s_rec + 3 * (B + 1u));  // [2][B] blocks met, bit by * kBlocks + bx
+    uint16_t* s_list = reinterpret_cast<uint16_t*>(s_hit + 2u * B);       // [groups][B + 4] byte offsets
+
+    const uint32_t row = blockIdx.x / (C * tiles_x), in_row = blockIdx.x - row * (C * tiles_x);
+    const uint32_t cam = in_row / tiles_x, tx = in_row - cam * tiles_x;
+    const uint32_t ty = (row & 1u) ? (tiles_y - 1u - row) / 2u : (tiles_y + row) / 2u;
+    const uint32_t n_tiles = tiles_x * tiles_y, key = cam * n_tiles + ty * tiles_x + tx;
+    const uint32_t ox = tx * kT, oy = ty * kT;
+    if (ox >= width || oy >= height) {
+        if (loss.target != nullptr && threadIdx.x == 0) loss.partials[key] = 0.0;
+        return;
+    }
+    const uint32_t vx = min(kT, width - ox), vy = min(kT, height - oy);
+    const int32_t start = offsets[key];
+    const int32_t n_total = n_dev != nullptr ? int32_t(*n_dev) : n_isects;
+    const int32_t end = (key + 1 == C * n_tiles) ? n_total : offsets[key + 1];
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, group = lane / kGroup, l = lane % kGroup;
+
+    // The warp's first block, this group's block and this lane's pixels.
+    const uint32_t wx = (warp % (kBlocks / kAcross)) * kAcross, wy = (warp / (kBlocks / kAcross)) * kDown;
+    const uint32_t lx = (wx + group % kAcross) * kBlock + l % kBlock, ly = (wy + group / kAcross) * kBlock + l / kBlock;
+    const float px = static_cast<float>(ox + lx) + 0.5f, fy = static_cast<float>(oy + ly) + 0.5f;
+    float2 py[kP], acc[kP], accv[kP];
+#pragma unroll
+    for (int k = 0; k < kP; ++k) {
+        py[k] = make_float2(fy + 4.f * static_cast<float>(k), fy + 4.f * static_cast<float>(k) + 2.f);
+        acc[k] = accv[k] = splat2(0.f);
+    }
+    uint16_t* lists = s_list + warp * kLists * (B + 4u);
+
+    // The padding record: sigma = 0 (d^2 = 0) with o mu = 0, so alpha = 0.
+    if (t < 3u) s_rec[t * (B + 1u) + B] = Rec2D<float>{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 1.f, 0.f};
+    const int32_t count = end - start;
+    const int32_t n_batches = count > 0 ? (count + int32_t(B) - 1) / int32_t(B) : 0;
+    auto load = [&](int32_t bi, uint32_t stage) {
+        for (uint32_t i = t; i < B; i += kThreads) {
+            const int32_t idx = start + bi * int32_t(B) + int32_t(i);
+            if (idx < end) gather_record(s_rec + stage * (B + 1u) + i, records + flatten_ids[idx]);
+        }
+        cp_async_commit();
+    };
+    if (n_batches > 0) load(0, 0);
+    for (int32_t bi = 0; bi < n_batches; ++bi) {
+        if (bi + 1 < n_batches) {
+            load(bi + 1, uint32_t(bi + 1) % 3u);
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
+        }
+        // A thread rewrites only records it copied itself: no barrier before this.
+        Rec2D<float>* buf = s_rec + (uint32_t(bi) % 3u) * (B + 1u);
+        uint32_t* hit = s_hit + (uint32_t(bi) & 1u) * B;
+        const int32_t batch = min(int32_t(B), count - bi * int32_t(B));
+        bool odd = false;
+        for (int32_t i = int32_t(t); i < batch; i += int32_t(kThreads)) {
+            Rec2D<float> rec = buf[i];
+            uint32_t x0 = 0u, x1 = vx - 1u, y0 = 0u, y1 = vy - 1u, mask = 0u;
+            bool bounded;
+            if (clip_to_record<float, kBeta>(rec, ox, oy, x0, x1, y0, y1, bounded)) {
+                const uint32_t line = (2u << (x1 / kBlock)) - (1u << (x0 / kBlock));
+                for (uint32_t y = y0 / kBlock; y <= y1 / kBlock; ++y) mask |= line << (y * kBlocks);
+                odd = odd || !bounded;
+            }
+            hit[i] = mask;
+            const float q =
+                kVar ? uncertainties[uint32_t(flatten_ids[start + bi * int32_t(B) + i]) % N] : 0.f;
+            buf[i] = Rec2D<float>{rec.x, kBeta ? rec.y : -rec.y, kBeta ? rec.a : 0.5f * rec.a, rec.b,
+                                  kBeta ? rec.c : 0.5f * rec.c, rec.o * rec.mu, rec.beta, q};
+        }
+        const bool strict = __syncthreads_or(odd);
+        // The hits of the warp's blocks, in list order.
+        uint32_t n[kLists];
+#pragma unroll
+        for (uint32_t g = 0; g < kLists; ++g) n[g] = 0u;
+        for (int32_t base = 0; base < batch; base += 32) {
+            const uint32_t m = base + int32_t(lane) < batch ? hit[base + int32_t(lane)] >> (wy * kBlocks + wx) : 0u;
+            const uint16_t at = uint16_t((uint32_t(base) + lane) * sizeof(Rec2D<float>));
+#pragma unroll
+            for (uint32_t g = 0; g < kLists; ++g) {
+                const bool mine = (m >> ((g / kAcross) * kBlocks + g % kAcross)) & 1u;
+                const uint32_t who = __ballot_sync(0xffffffffu, mine);
+                if (mine) lists[g * (B + 4u) + n[g] + __popc(who & ((1u << lane) - 1u))] = at;
+                n[g] += __popc(who);
+            }
+        }
+        uint32_t longest = 0u;
+#pragma unroll
+        for (uint32_t g = 0; g < kLists; ++g) longest = max(longest, n[g]);
+        longest = (longest + 3u) & ~3u;
+#pragma unroll
+        for (uint32_t g = 0; g < kLists; ++g)
+            for (uint32_t i = n[g] + lane; i < longest; i += 32u)
+                lists[g * (B + 4u) + i] = uint16_t(B * sizeof(Rec2D<float>));
+        __syncwarp();
+        const char* base_rec = reinterpret_cast<const char*>(buf);
+        const uint2* list = reinterpret_cast<const uint2*>(lists + group * (B + 4u));
+        for (uint32_t e = 0; e < longest; e += 4u) {
+            const uint2 four = list[e / 4u];
+            const char* r[4] = {base_rec + (four.x & 0xffffu), base_rec + (four.x >> 16),
+                                base_rec + (four.y & 0xffffu), base_rec + (four.y >> 16)};
+            if (!strict) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) group_record<kBeta, kVar, false>(r[k], px, py, acc, accv);
+            } else {
+#pragma unroll 1
+                for (int k = 0; k < 4; ++k) group_record<kBeta, kVar, true>(r[k], px, py, acc, accv);
+            }
+        }
+        __syncwarp();  // the lists are rewritten for the next batch
+        // No block barrier here: three record buffers, two mask buffers.
+    }
+    const size_t pid = size_t(cam) * height * width + size_t(oy + ly) * width + (ox + lx);
+    double term = 0.0;
+#pragma unroll
+    for (int k = 0; k < 2 * kP; ++k) {
+        const size_t p = pid + size_t(2 * k) * width;
+        if (lx < vx && ly + 2u * uint32_t(k) < vy) {
+            const float value = (k & 1) ? acc[k / 2].y : acc[k / 2].x;
+            render[p] = value;
+            if (kVar) render_var[p] = (k & 1) ? accv[k / 2].y : accv[k / 2].x;
+            if (loss.target != nullptr) {
+                const float diff = value - loss.target[p];
+                float v;
+                if (loss.l1) {
+                    const float sgn = diff > 0.f ? 1.f : (diff < 0.f ? -1.f : 0.f);
+                    v = loss.scale * sgn / loss.numel;
+                    term += fabs(static_cast<double>(diff));
+                } else {
+                    v = diff * loss.scale;
+                    term += static_cast<double>(diff) * static_cast<double>(diff);
+                }
+                loss.v_render[p] = v;
+            }
+        }
+    }
+    if (loss.target != nullptr) {
+        // Fixed-order CTA sum.
+        term = warp_sum(term);
+        double* s_sum = reinterpret_cast<double*>(smem);
+        __syncthreads();  // the records are no longer read
+        if (lane == 0u) s_sum[warp] = term;
+        __syncthreads();
+        if (t == 0u) {
+            double w = 0.0;
+            for (uint32_t k = 0; k < kThreads / 32u; ++k) w += s_sum[k];
+            loss.partials[key] = w;
+        }
+    }
+}
+
 // --------------------------------------------------------------------------
 // Backward
 // --------------------------------------------------------------------------
@@ -1127,10 +1366,43 @@ inline int check_geom(const RasterGeom& g) {
     return R2S_OK;
 }
 
+template <bool kBeta, bool kVar, uint32_t kT, uint32_t kBlock>
+int launch_fwd_group(const RasterGeom& g, const Rec2D<float>* rec, const float* unc, const int32_t* offsets,
+                     const int32_t* ids, float* out, float* out_var, const ImageLossEpilogue<float>& loss,
+                     unsigned most, cudaStream_t stream) {
+    // At most `most` records a batch: longer batches even out the groups' lists, shorter ones leave room for more
+    // CTAs. Tile 16, ms with 64, 128, 192, 224, 256: 65,536 lists of 720 Gaussians 3.87, 3.52, 3.46, 3.49, 3.54;
+    // 295,000 lists of 480 Beta records 10.0, 8.3, 8.01, 8.03, 8.18; 1024 lists of 360 0.132, 0.105, 0.101, -, 0.095.
+    // Tile 8 (one warp a tile), 8192 lists x 4: 0.628, 0.665, 0.729, 0.812, 0.839.
+    unsigned batch = g.stage_batch < most ? (g.stage_batch < 1 ? 1u : g.stage_batch) : most;
+    batch = (batch + 3u) & ~3u;  // the hit lists are read four entries at a time
+    constexpr unsigned groups = (kT / kBlock) * (kT / kBlock), threads = groups * 2u * kBlock;
+    const size_t smem = 3 * size_t(batch + 1) * sizeof(Rec2D<float>) + 2 * size_t(batch) * sizeof(uint32_t) +
+                        size_t(groups) * (batch + 4) * sizeof(uint16_t);
+    R2S_TRY(allow_dynamic_smem(raster_fwd_group_kernel<kBeta, kVar, kT, kBlock>, smem));
+    raster_fwd_group_kernel<kBeta, kVar, kT, kBlock><<<g.tiles_x * g.tiles_y * g.C, threads, smem, stream>>>(
+        rec, unc, g.N, offsets, ids, int32_t(g.n_isects), g.n_dev, g.C, g.width, g.height, g.tiles_x, g.tiles_y, out,
+        out_var, batch, loss);
+    return check_launch("rasterize_to_pixels_fwd");
+}
+
 template <typename S, bool kBeta, bool kVar>
 int launch_fwd_p(const RasterGeom& g, const Rec2D<S>* rec, const S* unc, const int32_t* offsets,
                  const int32_t* ids, S* out, S* out_var, const ImageLossEpilogue<S>& loss, cudaStream_t stream) {
     if constexpr (std::is_same<S, float>::value) {
+        // Tiles of whole 4x4 (8, 16) or 8x8 (32) blocks take the group kernel. Pair kernel against it, ms: 16 views
+        // of 256^2, 40,000 Gaussians 0.246 / 0.138 (tile 8), 0.179 / 0.115 (16), 0.262 / 0.207 (32); 32 views of
+        // 384^2, 100,000 Beta 0.81 / 0.25, 0.364 / 0.240, 0.524 / 0.428. At tile 32 a few lists are better off
+        // with the pair kernel's 16 warps a tile (16 lists of 340: 0.042 / 0.050).
+        const uint64_t lists = uint64_t(g.tiles_x) * g.tiles_y * g.C;
+        if (lists < (uint64_t(1) << 31)) {
+            if (g.T == 8)
+                return launch_fwd_group<kBeta, kVar, 8, 4>(g, rec, unc, offsets, ids, out, out_var, loss, 64u, stream);
+            if (g.T == 16)
+                return launch_fwd_group<kBeta, kVar, 16, 4>(g, rec, unc, offsets, ids, out, out_var, loss, 224u, stream);
+            if (g.T == 32 && lists >= 512)
+                return launch_fwd_group<kBeta, kVar, 32, 8>(g, rec, unc, offsets, ids, out, out_var, loss, 256u, stream);
+        }
         // Two pixels per lane: warps of 8x8 pixels.
         const uint32_t blocks = ((g.T + 7) / 8) * ((g.T + 7) / 8);
         const unsigned nthreads = 32u * blocks;

@@ -49,7 +49,9 @@ __device__ __forceinline__ bool clip_to_record(const Rec2D<S>& r, uint32_t ox, u
     bounded = a > S(0) && c > S(0) && det > S(0) && tr * tr <= S(1000) * det;
     S reach = S(1.001);
     if (!kBeta) {
-        S s = log(fabs(r.o * r.mu)) + S(11.512925464970229);  // ln(1e5)
+        const S om = fabs(r.o * r.mu);
+        if (bounded && om == S(0)) return false;  // every alpha is zero
+        S s = log(om) + S(11.512925464970229);    // ln(1e5)
         s = s + S(1e-3) * fabs(s) + S(1e-3);
         if (bounded && isfinite(s) && s < S(0)) return false;
         bounded = bounded && isfinite(s);
