@@ -321,6 +321,11 @@ int r2s_image_loss_l1_bwd(int dtype, const void* prediction, const void* target,
  * fewer passes over HBM.
  */
 
+/* Line-integral factor of Beta primitives (_beta.py:10-49), B(1/2, g + 1) /
+ * sqrt(2 pi) for exponents g = betas [n] > 0, into ratio [n], and the derivative
+ * of its logarithm into log_grad [n]; either may be null. Evaluated in double. */
+int r2s_beta_path_factor(int dtype, const void* betas, uint32_t n, void* ratio, void* log_grad, void* stream);
+
 /* Projection + conic/mu + packing (explicit.py:160-170). Writes one 8-slot
  * record per (camera, primitive) -- x, y, a, b, c, density, mu, beta+1/2 --
  * into records [C,N,8], the tile rectangle rects [C,N,4] (uint16: x0, y0, x1, y1),

@@ -1,4 +1,7 @@
-"""Line-integral factor of Beta primitives (host-side, float64).
+"""Line-integral factor of Beta primitives as tensor operations (float64).
+
+The pipelines evaluate the same two functions by one kernel each
+(``r2s_beta_path_factor``); these serve any device and autograd.
 
 A Beta density (1 - d^2)^gamma integrated along a ray has the Gaussian path
 factor times B(1/2, gamma + 1) / sqrt(2 pi); the projected exponent is

@@ -32,7 +32,6 @@ from typing import Optional
 
 import torch
 
-from . import _beta
 from .cuda import _backend
 from .cuda import _wrapper as low
 
@@ -66,6 +65,22 @@ def _dtype(t: Tensor) -> int:
 
 def _ws(nbytes: int, device) -> Tensor:
     return torch.empty(max(int(nbytes), 1), dtype=torch.uint8, device=device)
+
+
+def beta_path_ratio(beta: Tensor) -> Tensor:
+    """``_beta.beta_path_ratio`` of a contiguous CUDA tensor, as one kernel."""
+    ratio = torch.empty_like(beta)
+    _backend.call("r2s_beta_path_factor", _dtype(beta), _ptr(beta), beta.numel(), _ptr(ratio), None,
+                  _stream(beta.device))
+    return ratio
+
+
+def beta_path_log_grad(beta: Tensor) -> Tensor:
+    """``_beta.beta_path_log_grad`` of a contiguous CUDA tensor, as one kernel."""
+    log_grad = torch.empty_like(beta)
+    _backend.call("r2s_beta_path_factor", _dtype(beta), _ptr(beta), beta.numel(), None, _ptr(log_grad),
+                  _stream(beta.device))
+    return log_grad
 
 
 class StageTimer:
@@ -258,7 +273,7 @@ def raster_forward(means, quats, scales, densities, viewmats, Ks, width, height,
     device = means.device
     c = viewmats.shape[0]
     covars, _ = low.parameter_transform_fwd(quats, scales)
-    ratio = _beta.beta_path_ratio(beta) if beta is not None else None
+    ratio = beta_path_ratio(beta) if beta is not None else None
     records, offsets, isect_ids, flatten_ids, m, rects, cum = raster_intersections(
         means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps, radius_clip, tile_size,
         before_count)
@@ -293,7 +308,7 @@ def raster_vjp_state(means, quats, scales, densities, viewmats, Ks, width, heigh
     it reads them.
     """
     covars, _ = low.parameter_transform_fwd(quats, scales)
-    ratio = _beta.beta_path_ratio(beta) if beta is not None else None
+    ratio = beta_path_ratio(beta) if beta is not None else None
     records, rects, counts = _raster_project(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps,
                                              radius_clip, tile_size)
     return RasterState(covars, records, None, None, None, ratio, n_isects, width, height, tile_size,
@@ -348,7 +363,7 @@ def raster_backward(state: RasterState, means, quats, scales, densities, beta, u
                           stream)
     if v_unc is not None:
         _backend.call("r2s_sum_over_cameras", _dtype(means), _ptr(v_unc_cn), c, n, _ptr(v_unc), stream)
-    log_grad = _beta.beta_path_log_grad(beta) if beta is not None else None
+    log_grad = beta_path_log_grad(beta) if beta is not None else None
     v_means = means.new_empty((n, 3))
     v_quats = means.new_empty((n, 4))
     v_scales = means.new_empty((n, 3))

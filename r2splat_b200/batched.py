@@ -40,7 +40,7 @@ from typing import Optional, Sequence
 
 import torch
 
-from . import _beta
+from . import _fused
 from .cuda import _backend
 
 Tensor = torch.Tensor
@@ -217,7 +217,7 @@ class FitScene:
 
     def _project(self, stream):
         d = _dt(self.means)
-        self.ratio = _beta.beta_path_ratio(self.beta) if self.beta is not None else None
+        self.ratio = _fused.beta_path_ratio(self.beta) if self.beta is not None else None
         _backend.call("r2s_raster_project", d, _p(self.means), _p(self.covars), _p(self.densities), _p(self.beta),
                       _p(self.ratio), _p(self.viewmats), _p(self.Ks), self.c, self.n, self.width, self.height,
                       float(self.cfg.eps), float(self.cfg.eps), float(self.radius_clip), self.cfg.tile, self.tx,
@@ -269,7 +269,7 @@ class FitScene:
             _backend.call("r2s_raster_record_bwd", d, _p(self.records), _p(self.rects), None, beta_flag, 0,
                           _p(self.v_image), None, self.c, self.n, self.width, self.height, self.cfg.tile,
                           _p(self.grads2d), None, None, s)
-            log_grad = _beta.beta_path_log_grad(self.beta) if self.beta is not None else None
+            log_grad = _fused.beta_path_log_grad(self.beta) if self.beta is not None else None
             g = self.g_raster
             _backend.call("r2s_raster_chain_bwd", d, _p(self.means), _p(self.quats), _p(self.scales),
                           _p(self.covars), _p(self.beta), _p(self.ratio), _p(log_grad), _p(self.viewmats),

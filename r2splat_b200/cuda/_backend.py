@@ -72,6 +72,7 @@ SIGNATURES: dict[str, tuple] = {
     "r2s_volume_loss_fwd_bwd": (I32, [I32, P, P, U32, U32, U32, U32, F32, P, P, P, P, P, SZ, P]),
     "r2s_image_loss_l1_fwd": (I32, [I32, P, P, U32, U32, U32, F32, P, P, P, P, SZ, P]),
     "r2s_image_loss_l1_bwd": (I32, [I32, P, P, P, U32, U32, U32, F32, P, P]),
+    "r2s_beta_path_factor": (I32, [I32, P, U32, P, P, P]),
     "r2s_raster_project": (I32, [I32, P, P, P, P, P, P, P, U32, U32, U32, U32, F32, F64, F32, U32, U32, U32,
                                  P, P, P, P]),
     "r2s_raster_emit": (I32, [P, U32, U32, U32, U32, P, I64, P, P, P, P, SZ, P]),
