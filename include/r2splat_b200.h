@@ -75,11 +75,28 @@ typedef struct {
 } r2s_value_check;
 int r2s_check_values(int dtype, const r2s_value_check* checks, uint32_t n_checks, uint32_t* flags,
                      void* stream);
+/* The same checks, marking check c in byte bit of host_flags (32 bytes of pinned host memory, cleared
+ * by the call). *done receives an event recorded after them, for r2s_wait_done; host_flags must stay
+ * allocated until that returns. */
+int r2s_check_values_host(int dtype, const r2s_value_check* checks, uint32_t n_checks, uint8_t* host_flags,
+                          void** done, void* stream);
+
+/* Copies one device count to *host (pinned, kept until r2s_wait_done(*done) returns). */
+int r2s_read_count(const int64_t* count, int64_t* host, void** done, void* stream);
+
+/* Waits for the event of r2s_check_values_host / r2s_read_count and frees it. Call once. */
+int r2s_wait_done(void* done);
+
+/* dst[i] = values[i] in the dtype, for at most R2S_MAX_CONSTANTS host values, without stopping the
+ * stream as a copy from pageable memory does. */
+#define R2S_MAX_CONSTANTS 16
+int r2s_write_constants(int dtype, const double* values, uint32_t n, void* dst, void* stream);
 
 /* ---------------------------------------------------------------- geometry */
 
 /* Ops.h:419-422 parameter_transform_fwd_tensor.
- * quats [N,4] (wxyz, unnormalised), scales [N,3] -> covars [N,6], max_scales [N]. */
+ * quats [N,4] (wxyz, unnormalised), scales [N,3] -> covars [N,6], max_scales [N] (NULL: not
+ * written). */
 int r2s_parameter_transform_fwd(int dtype, const void* quats, const void* scales,
                                 void* covars, void* max_scales, uint32_t n, void* stream);
 

@@ -33,7 +33,6 @@ from typing import Optional
 import torch
 
 from .cuda import _backend
-from .cuda import _wrapper as low
 
 Tensor = torch.Tensor
 RASTER_TILE = 16
@@ -52,11 +51,10 @@ VOXEL_PACK_BUDGET_BYTES = VOXEL_SLOT_BUDGET_BYTES
 
 
 def _ptr(t: Optional[Tensor]):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
-def _stream(device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+_stream = _backend.stream_handle
 
 
 def _dtype(t: Tensor) -> int:
@@ -65,6 +63,29 @@ def _dtype(t: Tensor) -> int:
 
 def _ws(nbytes: int, device) -> Tensor:
     return torch.empty(max(int(nbytes), 1), dtype=torch.uint8, device=device)
+
+
+def _covariances(quats: Tensor, scales: Tensor) -> Tensor:
+    """Packed covariances [N,6] of validated (contiguous, same device and dtype) quats and scales."""
+    covars = quats.new_empty((quats.shape[0], 6))
+    _backend.call("r2s_parameter_transform_fwd", _dtype(quats), _ptr(quats), _ptr(scales), _ptr(covars), None,
+                  quats.shape[0], _stream(quats.device))
+    return covars
+
+
+def _read_total(cum: Tensor, before=None) -> int:
+    """The last entry of an inclusive scan. The copy is enqueued first, then ``before`` runs (it waits for work queued
+    earlier), so the device is never idle between the two waits."""
+    host = torch.empty(1, dtype=torch.int64, pin_memory=True)
+    done = ctypes.c_void_p()
+    _backend.call("r2s_read_count", _ptr(cum) + 8 * (cum.numel() - 1), _ptr(host), ctypes.byref(done),
+                  _stream(cum.device))
+    try:
+        if before is not None:
+            before()
+    finally:
+        _backend.call("r2s_wait_done", done)  # the copy writes the pinned word until here
+    return ctypes.c_int64.from_address(_ptr(host)).value
 
 
 def beta_path_ratio(beta: Tensor) -> Tensor:
@@ -177,9 +198,7 @@ def raster_intersections(means, covars, densities, beta, ratio, viewmats, Ks, wi
     records, rects, counts = _raster_project(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps,
                                              radius_clip, tile_size)
     cum = _raster_scan(counts)
-    if before_count is not None:
-        before_count()
-    m = int(cum[-1].item())
+    m = _read_total(cum, before_count)
     isect_ids, flatten_ids, offsets = _raster_lists(rects, cum, m, width, height, tile_size)
     return records, offsets, isect_ids, flatten_ids, m, rects, cum
 
@@ -272,7 +291,7 @@ def raster_forward(means, quats, scales, densities, viewmats, Ks, width, height,
     """
     device = means.device
     c = viewmats.shape[0]
-    covars, _ = low.parameter_transform_fwd(quats, scales)
+    covars = _covariances(quats, scales)
     ratio = beta_path_ratio(beta) if beta is not None else None
     records, offsets, isect_ids, flatten_ids, m, rects, cum = raster_intersections(
         means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps, radius_clip, tile_size,
@@ -307,7 +326,7 @@ def raster_vjp_state(means, quats, scales, densities, viewmats, Ks, width, heigh
     ``n_isects`` is the forward's intersection count of the same inputs; the VJP rebuilds the tile lists from it where
     it reads them.
     """
-    covars, _ = low.parameter_transform_fwd(quats, scales)
+    covars = _covariances(quats, scales)
     ratio = beta_path_ratio(beta) if beta is not None else None
     records, rects, counts = _raster_project(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps,
                                              radius_clip, tile_size)
@@ -319,11 +338,11 @@ def voxel_vjp_state(means, quats, scales, densities, shape, extent, center, beta
                     tile_size=VOXEL_TILE):
     """What the voxel VJP reads (covariances, records, voxel-space means and radii, layer scan),
     rebuilt without the volume: the projection and the layer counts, no intersection lists or sort."""
-    covars, _ = low.parameter_transform_fwd(quats, scales)
+    covars = _covariances(quats, scales)
     records, means_v, radii, _, _ = _voxel_project(means, covars, densities, beta, uncertainty, extent, center,
                                                    shape, eps, radius_clip, tile_size)
     layer_cum = _layer_scan(means_v, radii, shape, tile_size)
-    n_items = int(layer_cum[-1].item()) if layer_cum.numel() else 0
+    n_items = _read_total(layer_cum) if layer_cum.numel() else 0
     return VoxelState(covars, records, None, None, None, 0, tuple(shape), tile_size, means_v, radii, None,
                       layer_cum, n_items)
 
@@ -435,9 +454,7 @@ def voxel_intersections(means, covars, densities, beta, uncertainty, extent, cen
     lib = _backend.library()
     records, means_v, radii, _, cum = _voxel_project(means, covars, densities, beta, uncertainty, extent, center,
                                                      shape, eps, radius_clip, tile_size)
-    if before_count is not None:
-        before_count()
-    m = int(cum[-1].item())
+    m = _read_total(cum, before_count)
     isect_ids = torch.empty((m,), dtype=torch.int64, device=device)
     flatten_ids = torch.empty((m,), dtype=torch.int32, device=device)
     offsets = torch.empty((tz, ty, tx), dtype=torch.int32, device=device)
@@ -478,7 +495,7 @@ def voxel_forward(means, quats, scales, densities, shape, extent, center, beta, 
                   tile_size=VOXEL_TILE, before_count=None):
     device = means.device
     depth, height, width = shape
-    covars, _ = low.parameter_transform_fwd(quats, scales)
+    covars = _covariances(quats, scales)
     records, offsets, isect_ids, flatten_ids, m, means_v, radii, tile_cum = voxel_intersections(
         means, covars, densities, beta, uncertainty, extent, center, shape, eps, radius_clip, tile_size,
         before_count)
@@ -521,7 +538,7 @@ def voxel_backward(state: VoxelState, means, quats, scales, beta, uncertainty, e
     list_free = state.offsets is None or slot_bytes > VOXEL_SLOT_BUDGET_BYTES
     if list_free and state.layer_cum is None:
         state.layer_cum = _layer_scan(state.means_v, state.radii, state.shape, state.tile_size)
-        state.n_items = int(state.layer_cum[-1].item()) if n else 0
+        state.n_items = _read_total(state.layer_cum) if n else 0
     with _stage("voxel_render_bwd"):
         if not list_free:
             # Tile-parallel over the forward's sorted lists, one slot per (tile, primitive) pair.

@@ -20,10 +20,13 @@ import contextlib
 import ctypes
 import math
 import threading
+from array import array
 from numbers import Integral, Real
 from typing import Optional, Sequence, Union
 
 import torch
+
+from .cuda import _backend
 
 Tensor = torch.Tensor
 INT32_MAX = 2**31 - 1
@@ -46,33 +49,28 @@ class _ValueChecks:
         self._launched = None
 
     def launch(self) -> None:
-        """Enqueues the queued checks: one kernel per (device, dtype, 32 checks) and an
-        asynchronous copy of its flag word to pinned host memory, followed by an event."""
+        """Enqueues the queued checks: one kernel per (device, dtype, 32 checks), which marks
+        failures in pinned host memory, followed by an event."""
         items, self.items = self.items, []
         live = [(i, item) for i, item in enumerate(items) if item[0].numel() > 0]
         groups: dict = {}
         for index, item in live:
             groups.setdefault((item[0].device, item[0].dtype), []).append((index, item))
-        from .cuda import _backend  # late import: the loader imports nothing from here
-
-        words = []
+        words: list = []
+        self._launched = (items, words)
         for (device, dtype), group in groups.items():
             for start in range(0, len(group), 32):
                 chunk = group[start:start + 32]
-                table = (_ValueCheck * len(chunk))()
+                table = array("Q")  # r2s_value_check: data, count, kind | bit << 32
                 for bit, (_, (tensor, kind, _, _)) in enumerate(chunk):
-                    table[bit] = _ValueCheck(tensor.data_ptr(), tensor.numel() // _ELEMENT_SIZE[kind], kind, bit)
+                    table.extend((tensor.data_ptr(), tensor.numel() // _ELEMENT_SIZE[kind], kind | bit << 32))
+                host = torch.empty(32, dtype=torch.uint8, pin_memory=True)
+                done = ctypes.c_void_p()
                 with torch.cuda.device(device):
-                    stream = torch.cuda.current_stream(device)
-                    flags = torch.empty(1, dtype=torch.int32, device=device)
-                    _backend.call("r2s_check_values", 0 if dtype == torch.float32 else 1, table, len(chunk),
-                                  flags.data_ptr(), stream.cuda_stream)
-                    host = torch.empty(1, dtype=torch.int32, pin_memory=True)
-                    host.copy_(flags, non_blocking=True)
-                    done = torch.cuda.Event()
-                    done.record(stream)
+                    _backend.call("r2s_check_values_host", 0 if dtype == torch.float32 else 1,
+                                  table.buffer_info()[0], len(chunk), host.data_ptr(), ctypes.byref(done),
+                                  _backend.stream_handle(device))
                 words.append(([index for index, _ in chunk], host, done))
-        self._launched = (items, words)
 
     def resolve(self):
         """Waits for the launched checks only (work queued after them keeps running);
@@ -82,14 +80,24 @@ class _ValueChecks:
         items, words = self._launched
         self._launched = None
         failed: set = set()
-        for indices, host, done in words:
-            done.synchronize()
-            word = int(host[0])
-            failed.update(index for bit, index in enumerate(indices) if word >> bit & 1)
+        while words:
+            indices, host, done = words.pop()
+            _backend.call("r2s_wait_done", done)
+            marks = ctypes.string_at(host.data_ptr(), len(indices))
+            if any(marks):
+                failed.update(index for mark, index in zip(marks, indices) if mark)
         for index, (_, _, exc_type, message) in enumerate(items):
             if index in failed:
                 return exc_type(message)
         return None
+
+    def __del__(self):
+        # A launched kernel may still mark its pinned bytes: they are kept until it is done.
+        if self._launched is not None:
+            try:
+                self.resolve()
+            except Exception:  # a failed wait (the context is lost): nothing is left to protect
+                pass
 
     def first_failure(self):
         """Evaluates the queued checks; returns the first failing one's exception, or None."""
@@ -194,9 +202,23 @@ def _constant(name: str, value: Tensor) -> Tensor:
     return value
 
 
+def _upload(value: Sequence[float], reference: Tensor) -> Tensor:
+    """``torch.as_tensor(value)`` with the reference's dtype and device. Plain numbers of ordinary size travel as
+    kernel arguments: a copy from pageable memory would wait for all work queued on the stream."""
+    if (isinstance(value, (tuple, list)) and 0 < len(value) <= 16
+            and all(type(entry) in (int, float) and abs(entry) < 1e30 for entry in value)):
+        result = reference.new_empty((len(value),))
+        with torch.cuda.device(result.device):
+            _backend.call("r2s_write_constants", 0 if result.dtype == torch.float32 else 1,
+                          (ctypes.c_double * len(value))(*value), len(value), result.data_ptr(),
+                          _backend.stream_handle(result.device))
+        return result
+    return torch.as_tensor(value, device=reference.device, dtype=reference.dtype)
+
+
 def _vector(name: str, value: Union[Tensor, Sequence[float]], reference: Tensor) -> Tensor:
     if not isinstance(value, Tensor):
-        value = torch.as_tensor(value, device=reference.device, dtype=reference.dtype)
+        value = _upload(value, reference)
     return _constant(name, _tensor(name, value, (3,), reference))
 
 

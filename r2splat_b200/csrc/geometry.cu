@@ -24,7 +24,7 @@ __global__ void parameter_transform_fwd_kernel(const S* __restrict__ quats, cons
     covariance_from_parameters(q, s, cov, ms);
 #pragma unroll
     for (int k = 0; k < 6; ++k) covars[size_t(i) * 6 + k] = cov[k];
-    max_scales[i] = ms;
+    if (max_scales != nullptr) max_scales[i] = ms;
 }
 
 template <typename S>

@@ -33,6 +33,10 @@ SIGNATURES: dict[str, tuple] = {
     "r2s_sfu_peak_probe": (I32, [P, U32, U32, I32, P]),
     "r2s_launch_count": (U64, []),
     "r2s_check_values": (I32, [I32, P, U32, P, P]),
+    "r2s_check_values_host": (I32, [I32, P, U32, P, P, P]),
+    "r2s_read_count": (I32, [P, P, P, P]),
+    "r2s_wait_done": (I32, [P]),
+    "r2s_write_constants": (I32, [I32, P, U32, P, P]),
     "r2s_parameter_transform_fwd": (I32, [I32, P, P, P, P, U32, P]),
     "r2s_parameter_transform_bwd": (I32, [I32, P, P, P, P, P, U32, P]),
     "r2s_world_to_image_projection_fwd": (I32, [I32, P, P, P, P, U32, U32, U32, U32, F32, F32, P, P, P, P]),
@@ -133,6 +137,7 @@ SIGNATURES: dict[str, tuple] = {
 
 _lock = threading.Lock()
 _lib = None
+_cuda_seen = False  # torch.cuda.is_available() has been true
 _load_error: str | None = None
 
 
@@ -164,7 +169,7 @@ def _load():
 
 def library():
     """The loaded ctypes library; raises RuntimeError when unavailable."""
-    lib = _load()
+    lib = _lib if _lib is not None else _load()
     if lib is None:
         raise RuntimeError(_load_error)
     return lib
@@ -180,13 +185,31 @@ def is_cuda_available() -> bool:
 
 def call(name: str, *args) -> None:
     """Calls a C entry point and converts a nonzero status to RuntimeError."""
+    global _cuda_seen
     lib = library()
-    if not torch.cuda.is_available():
-        raise RuntimeError("r2splat_b200 operators require a CUDA device")
+    if not _cuda_seen:
+        if not torch.cuda.is_available():
+            raise RuntimeError("r2splat_b200 operators require a CUDA device")
+        _cuda_seen = True
     status = getattr(lib, name)(*args)
     if status != 0:
         message = lib.r2s_last_error().decode(errors="replace")
         raise RuntimeError(f"{name[4:]}: {message}")
 
 
-__all__ = ["SIGNATURES", "call", "is_cuda_available", "is_library_loadable", "library", "library_path"]
+def stream_handle(device: torch.device) -> int:
+    """The device's current stream as an integer handle (torch.cuda.current_stream(device).cuda_stream without the
+    stream object: 0.1 against 2.4 us, some 30 times per fitting step)."""
+    return _raw_stream(device.index if device.index is not None else torch.cuda.current_device())
+
+
+def _stream_object_handle(index: int) -> int:
+    return torch.cuda.current_stream(index).cuda_stream
+
+
+# The accessor torch's own compiled graphs call; older or newer torch without it takes the public one.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", _stream_object_handle)
+
+
+__all__ = ["SIGNATURES", "call", "is_cuda_available", "is_library_loadable", "library", "library_path",
+           "stream_handle"]

@@ -219,3 +219,51 @@ def test_finite_check_vector_path_positions(device, dtype):
                   torch.cuda.current_stream(device).cuda_stream)
     word = int(flags.item()) & 0xFFFFFFFF
     assert word == (1 << len(views)) - 2  # every bit but the all-finite tensor's
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_host_marks_name_the_failing_checks(device, dtype, offset):
+    """The pinned-memory marks: every byte of a clean batch stays 0, and a bad last element marks its check alone
+    (aligned and unaligned views, 32 checks, sizes around the vector width and the block)."""
+    import ctypes
+
+    from r2splat_b200._validation import FINITE, _ValueCheck
+    from r2splat_b200.cuda import _backend
+
+    sizes = ([1, 2, 3, 4, 5, 255, 256, 257, 1023, 4096, 300_001] * 3)[:32]
+    views = [torch.zeros(n + offset, device=device, dtype=dtype)[offset:] for n in sizes]
+    table = (_ValueCheck * len(views))()
+    for bit, view in enumerate(views):
+        table[bit] = _ValueCheck(view.data_ptr(), view.numel(), FINITE, bit)
+    host = torch.full((32,), 7, dtype=torch.uint8, pin_memory=True)
+    for bad in (None, 0, 10, 31):
+        if bad is not None:
+            views[bad][-1] = float("inf")
+        done = ctypes.c_void_p()
+        _backend.call("r2s_check_values_host", 0 if dtype == torch.float32 else 1, table, len(views),
+                      host.data_ptr(), ctypes.byref(done), torch.cuda.current_stream(device).cuda_stream)
+        _backend.call("r2s_wait_done", done)
+        assert host.tolist() == [int(i == bad) for i in range(32)]
+        if bad is not None:
+            views[bad][-1] = 0.0
+    with pytest.raises(RuntimeError, match="non-null"):
+        _backend.call("r2s_check_values_host", 0, table, 1, None, ctypes.byref(done), None)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("value", [(0.1, 2, -3.7e-20), [1.0], list(range(16)), (1e31, 1.0, 2.0), (True, 1, 2)])
+def test_uploaded_constants_are_those_of_as_tensor(device, dtype, value):
+    from r2splat_b200._validation import _upload
+
+    like = torch.empty(0, device=device, dtype=dtype)
+    assert torch.equal(_upload(value, like), torch.as_tensor(value, device=device, dtype=dtype))
+
+
+def test_read_total_waits_even_if_the_pending_checks_fail(device):
+    from r2splat_b200 import _fused
+
+    cum = torch.arange(1, 1000, device=device).cumsum(0)
+    assert _fused._read_total(cum) == int(cum[-1])
+    with pytest.raises(ValueError, match="pending"):
+        _fused._read_total(cum, lambda: (_ for _ in ()).throw(ValueError("pending")))
