@@ -250,13 +250,6 @@ __device__ __forceinline__ S mul_rn(S a, S b) {
     }
 }
 
-// 1.0f when a > b, else 0.0f (also 0.0f when either is NaN), as one PTX set.
-__device__ __forceinline__ float gt_mask(float a, float b) {
-    float m;
-    asm("set.gt.f32.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
-    return m;
-}
-
 // Raises a kernel's dynamic shared-memory limit when a launch needs more than
 // the default 48 KB in all (its dynamic bytes plus `static_bytes` of static
 // shared memory).

@@ -914,17 +914,20 @@ __constant__ uint32_t c_div_magic[33] = {
 // l = lane % kLanes evaluates two samples per step, k and k + kLanes of the
 // row-major box order (k = l + 2 kLanes it), so one FADD2/FMUL2/FFMA2 serves
 // both. iters is uniform over the warp.
-// Pixel centres are stepped exactly in float (integers + 0.5); the pixel's
-// element offset py * width + px - (width + 1) / 2 is formed exactly in float
-// as well and read out through the 2^23 bias (valid while width * height <
-// 2^22). The exponent e = -sigma log2(e) is evaluated from prescaled conic
+// The exponent e = -sigma log2(e) is evaluated from prescaled conic
 // coefficients as dx (a' dx + b' dy) + c' dy^2, so vis = 2^e. A sample counts
 // when e <= 0 (sigma >= 0) and e >= e_min, e_min = log2(1e-5 / |o mu|)
 // (|alpha| >= 1e-5): the reference's two decisions, taken on the exponent.
 // With w = -g alpha = -(o mu) g vis, the walk sums g vis and its moments and
 // scales them by -(o mu) once: part[0..4] are S0..S4 and part[5] = S5 of
 // vjp_sample.
-template <uint32_t kLanes = 32u>
+// kTest = false leaves out e <= 0 (a bounded conic's rounded sigma is never
+// negative, see clip_to_record). What bounds the walk is the FMA pipe, which
+// takes two to three cycles per packed operation, so the element offsets are
+// stepped as integers and the row wrap is predicated scalar arithmetic: 18
+// packed operations a step instead of 22. Pixel centres are stepped exactly in
+// float (integers + 0.5).
+template <uint32_t kLanes, bool kTest>
 __device__ __forceinline__ void record_walk_packed(const Rec2D<float>& r, float om, float e_min, const float* vimg,
                                                    uint32_t bx0, uint32_t by0, uint32_t bw, uint32_t barea,
                                                    uint32_t magic, uint32_t width, uint32_t iters, float (&part)[8]) {
@@ -935,33 +938,28 @@ __device__ __forceinline__ void record_walk_packed(const Rec2D<float>& r, float 
     const uint32_t ca = lane - ra * bw, cb = lane + kLanes - rb * bw;
     float2 px = make_float2(static_cast<float>(bx0 + ca) + 0.5f, static_cast<float>(bx0 + cb) + 0.5f);
     float2 py = make_float2(static_cast<float>(by0 + ra) + 0.5f, static_cast<float>(by0 + rb) + 0.5f);
-    const float x_end = static_cast<float>(bx0 + bw);
+    uint32_t offa = (by0 + ra) * width + bx0 + ca, offb = (by0 + rb) * width + bx0 + cb;
+    const uint32_t step = dq * width + dr, wrap_step = width - bw;
+    const float x_end = static_cast<float>(bx0 + bw), fbw = static_cast<float>(bw);
     const float2 step_x = splat2(static_cast<float>(dr)), step_y = splat2(static_cast<float>(dq));
-    const float2 neg_bw = splat2(-static_cast<float>(bw));
-    const float2 fw = splat2(static_cast<float>(width));
-    // 2^23 - (width + 1) / 2: exact in float for width < 2^22.
-    const float2 bias = splat2(8388608.0f - 0.5f * static_cast<float>(width) - 0.5f);
-    const uint64_t vbase = reinterpret_cast<uint64_t>(vimg) - uint64_t(0x4B000000u) * sizeof(float);
     const float2 nx = splat2(-r.x), ny = splat2(-r.y);
     const float2 qa = splat2(0.5f * r.a * kNegLog2e), qb = splat2(r.b * kNegLog2e);
     const float2 qc = splat2(0.5f * r.c * kNegLog2e);
     float2 acc0 = splat2(0.f), acc1 = acc0, acc2 = acc0, acc3 = acc0, acc4 = acc0, acc5 = acc0;
     uint32_t k = lane;
     // Two steps per loop trip: the second step's adjoint loads are issued with
-    // the first's (1.8 % off the CT VJP; four steps gained nothing more).
+    // the first's (without it the CT VJP takes 27 % longer; four steps at 80
+    // registers gained nothing more).
 #pragma unroll 2
     for (uint32_t it = 0; it < iters; ++it, k += 2u * kLanes) {
-        const float2 offb = add2(fma2(py, fw, px), bias);
-        const float* pa = reinterpret_cast<const float*>(vbase + uint64_t(__float_as_uint(offb.x)) * sizeof(float));
-        const float* pb = reinterpret_cast<const float*>(vbase + uint64_t(__float_as_uint(offb.y)) * sizeof(float));
-        const float ga = k < barea ? __ldg(pa) : 0.f;
-        const float gb = k + kLanes < barea ? __ldg(pb) : 0.f;
+        const float ga = k < barea ? __ldg(vimg + offa) : 0.f;
+        const float gb = k + kLanes < barea ? __ldg(vimg + offb) : 0.f;
         const float2 dx = add2(px, nx), dy = add2(py, ny);
         const float2 t = fma2(qa, dx, mul2(qb, dy));
         const float2 e = fma2(dx, t, mul2(mul2(qc, dy), dy));
         const float2 vis = make_float2(exp2f(e.x), exp2f(e.y));
-        const bool ka = !(e.x > 0.f || e.x < e_min);
-        const bool kb = !(e.y > 0.f || e.y < e_min);
+        const bool ka = !((kTest && e.x > 0.f) || e.x < e_min);
+        const bool kb = !((kTest && e.y > 0.f) || e.y < e_min);
         // Select after the product: a skipped sample may have vis = inf (e > 0).
         const float2 gvr = mul2(make_float2(ga, gb), vis);
         const float2 gv = make_float2(ka ? gvr.x : 0.f, kb ? gvr.y : 0.f);
@@ -972,13 +970,22 @@ __device__ __forceinline__ void record_walk_packed(const Rec2D<float>& r, float 
         acc3 = fma2(wx, dy, acc3);
         acc4 = fma2(wy, dy, acc4);
         acc5 = add2(acc5, gv);
-        // Advance both samples by 64 box positions: dq rows and dr columns,
+        // Advance both samples by 2 kLanes box positions: dq rows and dr columns,
         // plus one wrap where the column passes the box's width.
         px = add2(px, step_x);
         py = add2(py, step_y);
-        const float2 wrap = make_float2(gt_mask(px.x, x_end), gt_mask(px.y, x_end));
-        px = fma2(wrap, neg_bw, px);
-        py = add2(py, wrap);
+        offa += step;
+        offb += step;
+        if (px.x > x_end) {
+            px.x -= fbw;
+            py.x += 1.f;
+            offa += wrap_step;
+        }
+        if (px.y > x_end) {
+            px.y -= fbw;
+            py.y += 1.f;
+            offb += wrap_step;
+        }
     }
     const float nom = -om;
     part[0] = nom * (acc0.x + acc0.y);
@@ -1064,6 +1071,9 @@ __device__ __forceinline__ void store_record_adjoints(const Rec2D<S>& r, uint32_
     if (kVar && grp == 3u && v_unc != nullptr) v_unc[rid] = hi;
 }
 
+// Set in a record's magic (at most 2^16) when its conic is not bounded.
+constexpr uint32_t kUnbounded = 0x80000000u;
+
 // A record's walk constants, set up by the lane that loaded the record and
 // read by the whole warp from shared memory (broadcast loads).
 template <typename S>
@@ -1100,7 +1110,8 @@ __device__ __forceinline__ uint32_t warp_sort_ascending(uint32_t key) {
 // of the warp's records, so a step's records have boxes of about one size.
 // base is the warp's first record; var_q is null without the variance chain
 // term.
-template <typename S, bool kBeta, bool kVar, bool kAbs, uint32_t kLanes, bool kPackedWalk>
+template <typename S, bool kBeta, bool kVar, bool kAbs, uint32_t kLanes, bool kPackedWalk,
+          bool kTest>
 __device__ __forceinline__ void walk_record_groups(uint32_t sorted, uint32_t p, uint32_t p_end,
                                                    const RecordStage<S>* stage, size_t base, uint32_t N,
                                                    uint32_t width, uint32_t height, const S* v_render,
@@ -1134,8 +1145,8 @@ __device__ __forceinline__ void walk_record_groups(uint32_t sorted, uint32_t p, 
         S part[8];
         S g_ax = S(0), g_ay = S(0);
         if constexpr (kPackedWalk)
-            record_walk_packed<kLanes>(r, om, st.e_min, vimg, st.x0, st.y0, st.w, barea, st.magic, width, iters,
-                                       part);
+            record_walk_packed<kLanes, kTest>(r, om, st.e_min, vimg, st.x0, st.y0, st.w, barea,
+                                              st.magic & ~kUnbounded, width, iters, part);
         else
             record_walk_scalar<S, kBeta, kVar, kAbs, kLanes>(r, om, q, vimg, vvar, st.x0, st.y0, st.w, barea,
                                                              iters, width, part, g_ax, g_ay);
@@ -1158,18 +1169,25 @@ __device__ __forceinline__ void walk_record_groups(uint32_t sorted, uint32_t p, 
     }
 }
 
+// Blocks per SM the record VJP is compiled for: three (80 registers) for fp32. Two (122) or four (64, with spills for
+// the packed walk) are slower; the Beta variance form would take two on its own.
+template <typename S>
+constexpr int kRecBwdMinBlocks = sizeof(S) == 4 ? 3 : 0;
+
 template <typename S, bool kBeta, bool kVar, bool kAbs>
-__global__ void __launch_bounds__(kRecBwdThreads) raster_record_bwd_kernel(
+__global__ void __launch_bounds__(kRecBwdThreads, kRecBwdMinBlocks<S>) raster_record_bwd_kernel(
     const Rec2D<S>* __restrict__ records, const ushort4* __restrict__ rects, const S* __restrict__ var_q,
     uint32_t C, uint32_t N, uint32_t width, uint32_t height, uint32_t T, const S* __restrict__ v_render,
     const S* __restrict__ v_render_var, Rec2D<S>* __restrict__ grads, S* __restrict__ v_abs,
-    S* __restrict__ v_unc) {
+    S* __restrict__ v_unc, uint32_t batches) {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t warps_per_block = blockDim.x >> 5;
     const size_t total = size_t(C) * N;
-    const size_t group_stride = size_t(gridDim.x) * warps_per_block * 32u;
+    // A block takes `batches` runs of kRecBwdThreads consecutive records.
+    const size_t first = size_t(blockIdx.x) * batches * kRecBwdThreads;
+    const size_t last = min(total, first + size_t(batches) * kRecBwdThreads);
     const bool chain_var = kVar && var_q != nullptr;
-    // The packed two-samples-per-lane walk serves the plain Gaussian VJP.
+    // The packed two-samples-per-lane walk serves the plain Gaussian VJP; images of 2^22 pixels and more keep the scalar
+    // walk's sums.
     constexpr bool kPacked = std::is_same<S, float>::value && !kBeta && !kVar && !kAbs;
     const bool packed = kPacked && v_render != nullptr && uint64_t(width) * height < (uint64_t(1) << 22);
     // Each warp takes 32 consecutive records at a time. Lane-parallel set-up:
@@ -1179,8 +1197,7 @@ __global__ void __launch_bounds__(kRecBwdThreads) raster_record_bwd_kernel(
     // broadcast loads.
     __shared__ RecordStage<S> s_stage[kRecBwdThreads];
     RecordStage<S>* stage = s_stage + (threadIdx.x & ~31u);
-    for (size_t base = (size_t(blockIdx.x) * warps_per_block + (threadIdx.x >> 5)) * 32u; base < total;
-         base += group_stride) {
+    for (size_t base = first + (threadIdx.x & ~31u); base < last; base += kRecBwdThreads) {
         const size_t my_rid = base + lane;
         Rec2D<S> mine;
         uint32_t x0 = 0u, y0 = 0u, w = 0u, area = 0u, magic = 0u;
@@ -1192,17 +1209,17 @@ __global__ void __launch_bounds__(kRecBwdThreads) raster_record_bwd_kernel(
             x0 = uint32_t(rect.x) * T;
             y0 = uint32_t(rect.y) * T;
             uint32_t x1 = min(uint32_t(rect.z) * T, width), y1 = min(uint32_t(rect.w) * T, height);
-            bool any = rect.z > rect.x && rect.w > rect.y && x0 < x1 && y0 < y1;
+            bool any = rect.z > rect.x && rect.w > rect.y && x0 < x1 && y0 < y1, bounded = false;
             mine = records[my_rid];
             if (any) {
                 x1 -= 1u;
                 y1 -= 1u;
-                any = clip_to_record<S, kBeta>(mine, 0u, 0u, x0, x1, y0, y1);
+                any = clip_to_record<S, kBeta>(mine, 0u, 0u, x0, x1, y0, y1, bounded);
             }
             if (any) {
                 w = x1 - x0 + 1u;
                 area = w * (y1 - y0 + 1u);
-                if (kPacked) magic = (65536u + w - 1u) / w;
+                if (kPacked) magic = (65536u + w - 1u) / w | (bounded ? 0u : kUnbounded);
             } else {
                 // No pixel can contribute: the record's adjoints are zero.
                 S* dst = reinterpret_cast<S*>(grads + my_rid);
@@ -1257,8 +1274,13 @@ __global__ void __launch_bounds__(kRecBwdThreads) raster_record_bwd_kernel(
             bool walked = false;
             if constexpr (kPacked) {
                 if (packed) {
-                    record_walk_packed(r, om, st.e_min, vimg, bx0, by0, bw, barea, st.magic, width,
-                                       (barea + 63u) >> 6, part);
+                    const uint32_t magic = st.magic & ~kUnbounded;  // st is the warp's one record
+                    if ((st.magic & kUnbounded) != 0u)
+                        record_walk_packed<32u, true>(r, om, st.e_min, vimg, bx0, by0, bw, barea, magic, width,
+                                                      (barea + 63u) >> 6, part);
+                    else
+                        record_walk_packed<32u, false>(r, om, st.e_min, vimg, bx0, by0, bw, barea, magic, width,
+                                                       (barea + 63u) >> 6, part);
                     walked = true;
                 }
             }
@@ -1297,12 +1319,23 @@ __global__ void __launch_bounds__(kRecBwdThreads) raster_record_bwd_kernel(
             const uint32_t n_quad = __popc(__ballot_sync(0xffffffffu, grouped && area <= quarter_area));
             if (n_group != 0u) {
                 const uint32_t sorted = warp_sort_ascending(grouped ? (area << 5) | lane : 0xffffffe0u | lane);
-                walk_record_groups<S, kBeta, kVar, kAbs, 8u, kPacked>(sorted, 0u, n_quad, stage, base, N, width, height,
-                                                             v_render, v_render_var, chain_var ? var_q : nullptr,
-                                                             grads, v_abs, v_unc);
-                walk_record_groups<S, kBeta, kVar, kAbs, 16u, kPacked>(sorted, n_quad, n_group, stage, base, N, width,
-                                                              height, v_render, v_render_var,
-                                                              chain_var ? var_q : nullptr, grads, v_abs, v_unc);
+                const S* q = chain_var ? var_q : nullptr;
+                // One choice for the warp's records (a choice per step costs the CT VJP 1.5 %).
+                if (kPacked && !__any_sync(0xffffffffu, grouped && (magic & kUnbounded) != 0u)) {
+                    walk_record_groups<S, kBeta, kVar, kAbs, 8u, kPacked, false>(
+                        sorted, 0u, n_quad, stage, base, N, width, height, v_render, v_render_var, q, grads, v_abs,
+                        v_unc);
+                    walk_record_groups<S, kBeta, kVar, kAbs, 16u, kPacked, false>(
+                        sorted, n_quad, n_group, stage, base, N, width, height, v_render, v_render_var, q, grads,
+                        v_abs, v_unc);
+                } else {
+                    walk_record_groups<S, kBeta, kVar, kAbs, 8u, kPacked, true>(
+                        sorted, 0u, n_quad, stage, base, N, width, height, v_render, v_render_var, q, grads, v_abs,
+                        v_unc);
+                    walk_record_groups<S, kBeta, kVar, kAbs, 16u, kPacked, true>(
+                        sorted, n_quad, n_group, stage, base, N, width, height, v_render, v_render_var, q, grads,
+                        v_abs, v_unc);
+                }
             }
         }
     }
@@ -1513,19 +1546,24 @@ int launch_record_bwd_t(const RasterGeom& g, const Rec2D<S>* rec, const ushort4*
                         const S* v_render, const S* v_render_var, Rec2D<S>* grads, S* v_abs, S* v_unc,
                         cudaStream_t stream) {
     const size_t total = size_t(g.C) * g.N;
-    const size_t warps_per_block = kRecBwdThreads / 32;
-    int device = 0, sms = 148, per_sm = 4;
+    int device = 0, sms = 148, per_sm = 3;
     if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, raster_record_bwd_kernel<S, kBeta, kVar, kAbs>,
                                                   kRecBwdThreads, 0);
-    // Persistent grid: exactly the resident blocks, each warp striding over
-    // records, so every warp takes the same number of records and none waits
-    // for a late wave.
-    size_t blocks = (total + warps_per_block - 1) / warps_per_block;
-    const size_t cap = size_t(sms > 0 ? sms : 148) * size_t(per_sm > 0 ? per_sm : 1);
-    if (blocks > cap) blocks = cap;
+    // The blocks are dispatched in record order as others finish, so the records in flight stay together in memory and
+    // slow batches even out. (Warps striding over all records drift apart: the Beta variance VJP of 500,000 primitives
+    // and 128 views of 768^2 took 18.6 ms that way, 145 us a view against 109 at 64 views, and takes 11.9 ms; the
+    // cone-beam one, 200,000 and 64 views of 512^2, 6.36 -> 5.74 ms with the walk's changes.) Two batches a block from
+    // four waves on, four from 64: fewer blocks to dispatch (four against one at 64 views: 11.9 / 12.4 and 5.80 / 5.86
+    // ms), which kernels that share the device also notice (four scenes of 40,000 and 16 views stepped as one graph:
+    // 1.133 ms with two, 1.141 with one); at 2.6 waves two batches leave a short last wave (0.227 / 0.205 ms).
+    const size_t wave = size_t(sms > 0 ? sms : 148) * size_t(per_sm > 0 ? per_sm : 1);
+    const size_t runs = (total + kRecBwdThreads - 1) / kRecBwdThreads;
+    const size_t batches = runs >= 64 * wave ? 4 : runs >= 4 * wave ? 2 : 1;
+    const size_t blocks = (runs + batches - 1) / batches;
     raster_record_bwd_kernel<S, kBeta, kVar, kAbs><<<unsigned(blocks), kRecBwdThreads, 0, stream>>>(
-        rec, rects, var_q, g.C, g.N, g.width, g.height, g.T, v_render, v_render_var, grads, v_abs, v_unc);
+        rec, rects, var_q, g.C, g.N, g.width, g.height, g.T, v_render, v_render_var, grads, v_abs, v_unc,
+        uint32_t(batches));
     return check_launch("raster_record_bwd");
 }
 
