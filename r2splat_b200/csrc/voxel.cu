@@ -1117,9 +1117,8 @@ __global__ void voxel_slot_reduce_kernel(const S* __restrict__ slots, const int6
     for (int i = 0; i < 4; ++i) out[i] = q == 0u ? acc[i] : q == 1u ? acc[4 + i] : q == 2u ? acc[8 + i] : S(0);
 }
 
-// Tile VJP of fp32 Gaussian records on 8^3 tiles without the variance branch
-// (the CT fit step's form), one lane per (tile, primitive) pair. The warp
-// walks the tile's 512 voxels in lockstep, z, then pairs of rows, then x; the
+// Tile VJP of fp32 Gaussian records on 8^3 tiles, one lane per (tile,
+// primitive) pair. The warp walks the tile's 512 voxels in lockstep, z, then pairs of rows, then x; the
 // voxel is the same for every lane, so its adjoint is one broadcast shared-
 // memory read for 32 records, and each lane sums its own record's moments
 // serially: no per-pair reduction across lanes, no box set-up. The whole tile
@@ -1133,18 +1132,104 @@ __global__ void voxel_slot_reduce_kernel(const S* __restrict__ slots, const int6
 // adds g vis, g vis d1 and g vis d1^2 to the row sums. A pair of rows folds
 // them with its d2 values, a z slab with its d3; the record's sums are then
 // the ones voxel_bwd_kernel forms (w = -o g vis), and the 12 values written
-// per pair are the same quantities in the same layout.
+// per pair are the same quantities in the same layout. With the variance
+// branch (kVar) g becomes g + 2 q o u vis for the variance adjoint u (nothing
+// added when detached), and o^2 sum u vis^2 is the uncertainty's adjoint.
+//
+// Bound by a step's latency as much as by its pipes (16 cycles of exponentials
+// and about 20 of packed FP32 a pair of samples): 128 registers and a whole z
+// slab unrolled beat more warps with fewer. Chunks whose records all have
+// bounded conics leave out e <= 0, which then holds. 200,000 primitives in
+// 256^3 (6.8 M pairs), kernel and slot sum: 1.91 -> 1.61 ms; 120,007 in 301 x
+// 263 x 277: 1.43 -> 1.21 ms (six blocks a SM at 80 registers, rows one by one
+// before). The variance branch, 50,021 in 150 x 173 x 201: 0.92 -> 0.40 ms (a warp
+// per record before).
 constexpr int kVoxLaneWarps = 4;
 constexpr int kVoxLaneThreads = kVoxLaneWarps * 32;
 
-template <bool kBulk>
-__global__ void __launch_bounds__(kVoxLaneThreads, 6) voxel_bwd_lanes_kernel(
-    const Rec3D<float>* __restrict__ records, const int32_t* __restrict__ offsets,
-    const int32_t* __restrict__ flatten_ids, VoxelGeom g, const float* __restrict__ v_volume,
-    Rec3D<float>* __restrict__ grads, VoxelSlots<float> sl) {
+// A lane's walk of the tile: the moments of g vis over the voxels that count.
+struct LaneSums {
+    // g vis d1^2, g vis d2^2, g vis d1 d2 and u vis^2, packed over the row pair.
+    float2 r11, r22, r12, ru;
+    // g vis, g vis d1, g vis d2 and the d3 moments.
+    float s0, s1, s2, s3, s13, s23, s33;
+};
+
+// s_g[(z * 4 + yp) * 8 + x] holds the adjoints of rows 2 yp and 2 yp + 1, s_u likewise (kVar). k2 = 2 q o.
+template <bool kVar, bool kTest>
+__device__ __forceinline__ LaneSums lane_walk(const float2* s_g, const float2* s_u, float4 q0, float4 q1, float4 q2,
+                                              float e_min, float k2, float fx, float fy, float fz) {
     constexpr uint32_t T = 8u;
-    // The tile's adjoint as row pairs: s_g[(z * 4 + yp) * 8 + x] = (g(z, 2 yp, x), g(z, 2 yp + 1, x)).
+    const float ry = q0.y, rz = q0.z;
+    const float2 qa = splat2(0.5f * q1.x * kVoxNegLog2e);
+    const float pl = q1.y * kVoxNegLog2e, ql3 = q1.z * kVoxNegLog2e;
+    const float hb = 0.5f * q1.w * kVoxNegLog2e, rl = q2.x * kVoxNegLog2e, hc = 0.5f * q2.y * kVoxNegLog2e;
+    const float2 d1_0 = splat2(fx - q0.x), one = splat2(1.f), kk = splat2(k2);
+    LaneSums r{};
+    for (uint32_t z = 0; z < T; ++z) {
+        const float d3 = (fz + static_cast<float>(z)) - rz;
+        const float qd3 = ql3 * d3, rd3 = rl * d3, cd3 = hc * d3 * d3;
+        float2 z0 = splat2(0.f), z1 = z0, z2 = z0;
+        const uint32_t base = z * (T * T / 2);
+#pragma unroll
+        for (uint32_t yp = 0; yp < T / 2; ++yp) {
+            const float fyp = fy + static_cast<float>(2u * yp);
+            const float2 d2 = make_float2(fyp - ry, (fyp + 1.f) - ry);
+            const float2 ql = make_float2(fmaf(pl, d2.x, qd3), fmaf(pl, d2.y, qd3));
+            const float2 qk = make_float2(fmaf(hb * d2.x, d2.x, fmaf(rd3, d2.x, cd3)),
+                                          fmaf(hb * d2.y, d2.y, fmaf(rd3, d2.y, cd3)));
+            float2 a1 = splat2(0.f), a2 = a1, a3 = a1;
+            float2 d1 = d1_0;
+#pragma unroll
+            for (uint32_t x = 0; x < T; ++x) {
+                float2 gg = s_g[base + yp * T + x];
+                const float2 e = fma2(fma2(qa, d1, ql), d1, qk);
+                const float2 vis = make_float2(exp2f(e.x), exp2f(e.y));
+                const bool ka = !((kTest && e.x > 0.f) || e.x < e_min);
+                const bool kb = !((kTest && e.y > 0.f) || e.y < e_min);
+                // Select after the products: a skipped sample may have vis = inf (e > 0).
+                if (kVar) {
+                    const float2 uv = mul2(s_u[base + yp * T + x], vis);
+                    gg = fma2(kk, uv, gg);
+                    const float2 uv2 = mul2(uv, vis);
+                    r.ru = add2(r.ru, make_float2(ka ? uv2.x : 0.f, kb ? uv2.y : 0.f));
+                }
+                const float2 gvr = mul2(gg, vis);
+                const float2 gv = make_float2(ka ? gvr.x : 0.f, kb ? gvr.y : 0.f);
+                a3 = add2(a3, gv);
+                const float2 gvd = mul2(gv, d1);
+                a1 = add2(a1, gvd);
+                a2 = fma2(gvd, d1, a2);
+                d1 = add2(d1, one);
+            }
+            z0 = add2(z0, a3);
+            z1 = add2(z1, a1);
+            r.r11 = add2(r.r11, a2);
+            const float2 gd2 = mul2(d2, a3);
+            z2 = add2(z2, gd2);
+            r.r22 = fma2(d2, gd2, r.r22);
+            r.r12 = fma2(d2, a1, r.r12);
+        }
+        const float g0 = z0.x + z0.y, g1 = z1.x + z1.y, g2 = z2.x + z2.y;
+        r.s0 += g0;
+        r.s1 += g1;
+        r.s2 += g2;
+        r.s3 = fmaf(d3, g0, r.s3);
+        r.s13 = fmaf(d3, g1, r.s13);
+        r.s23 = fmaf(d3, g2, r.s23);
+        r.s33 = fmaf(d3 * d3, g0, r.s33);
+    }
+    return r;
+}
+
+template <bool kVar, bool kBulk>
+__global__ void __launch_bounds__(kVoxLaneThreads, 4) voxel_bwd_lanes_kernel(
+    const Rec3D<float>* __restrict__ records, bool chain_var, const int32_t* __restrict__ offsets,
+    const int32_t* __restrict__ flatten_ids, VoxelGeom g, const float* __restrict__ v_volume,
+    const float* __restrict__ v_volume_var, Rec3D<float>* __restrict__ grads, VoxelSlots<float> sl) {
+    constexpr uint32_t T = 8u;
     __shared__ float2 s_g[T * T * T / 2];
+    __shared__ float2 s_u[kVar ? T * T * T / 2 : 1];
     const uint32_t n_tiles = g.tiles_x * g.tiles_y * g.tiles_z;
     const uint32_t key = blockIdx.x;
     const uint32_t tz = key / (g.tiles_x * g.tiles_y);
@@ -1161,13 +1246,20 @@ __global__ void __launch_bounds__(kVoxLaneThreads, 6) voxel_bwd_lanes_kernel(
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
     for (uint32_t p = t; p < T * T * T / 2; p += kVoxLaneThreads) {
         const uint32_t x = p & 7u, yp = (p >> 3) & 3u, z = p >> 5;
-        float ga = 0.f, gb = 0.f;
-        if (v_volume != nullptr && x < vx && z < vz) {
+        float ga = 0.f, gb = 0.f, ua = 0.f, ub = 0.f;
+        if (x < vx && z < vz) {
             const size_t vid = (size_t(oz + z) * g.dim1 + (oy + 2u * yp)) * g.dim2 + (ox + x);
-            if (2u * yp < vy) ga = v_volume[vid];
-            if (2u * yp + 1u < vy) gb = v_volume[vid + g.dim2];
+            if (2u * yp < vy) {
+                if (v_volume != nullptr) ga = v_volume[vid];
+                if (kVar) ua = v_volume_var[vid];
+            }
+            if (2u * yp + 1u < vy) {
+                if (v_volume != nullptr) gb = v_volume[vid + g.dim2];
+                if (kVar) ub = v_volume_var[vid + g.dim2];
+            }
         }
         s_g[p] = make_float2(ga, gb);
+        if (kVar) s_u[p] = make_float2(ua, ub);
     }
     __syncthreads();
 
@@ -1207,75 +1299,27 @@ __global__ void __launch_bounds__(kVoxLaneThreads, 6) voxel_bwd_lanes_kernel(
             q1 = __ldg(r4 + 1);
             q2 = __ldg(r4 + 2);
         }
-        const float ry = q0.y, rz = q0.z, opac = q0.w;
+        const float opac = q0.w;
         const float e_min = log2f(1e-6f / fabsf(opac));
-        const float2 qa = splat2(0.5f * q1.x * kVoxNegLog2e);
-        const float pl = q1.y * kVoxNegLog2e, ql3 = q1.z * kVoxNegLog2e;
-        const float hb = 0.5f * q1.w * kVoxNegLog2e, rl = q2.x * kVoxNegLog2e, hc = 0.5f * q2.y * kVoxNegLog2e;
-        const float2 d1_0 = splat2(fx - q0.x), one = splat2(1.f);
-        // Record sums: g vis d1^2, g vis d2^2, g vis d1 d2 (packed over the row pair),
-        // then g vis, g vis d1, g vis d2 and the d3 moments.
-        float2 r11 = splat2(0.f), r22 = r11, r12 = r11;
-        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f, s13 = 0.f, s23 = 0.f, s33 = 0.f;
-        for (uint32_t z = 0; z < T; ++z) {
-            const float d3 = (fz + static_cast<float>(z)) - rz;
-            const float qd3 = ql3 * d3, rd3 = rl * d3, cd3 = hc * d3 * d3;
-            float2 z0 = splat2(0.f), z1 = z0, z2 = z0;
-            const float2* gz = s_g + z * (T * T / 2);
-#pragma unroll 1
-            for (uint32_t yp = 0; yp < T / 2; ++yp) {
-                const float fyp = fy + static_cast<float>(2u * yp);
-                const float2 d2 = make_float2(fyp - ry, (fyp + 1.f) - ry);
-                const float2 ql = make_float2(fmaf(pl, d2.x, qd3), fmaf(pl, d2.y, qd3));
-                const float2 qk = make_float2(fmaf(hb * d2.x, d2.x, fmaf(rd3, d2.x, cd3)),
-                                              fmaf(hb * d2.y, d2.y, fmaf(rd3, d2.y, cd3)));
-                float2 a1 = splat2(0.f), a2 = a1, a3 = a1;
-                float2 d1 = d1_0;
-#pragma unroll
-                for (uint32_t x = 0; x < T; ++x) {
-                    const float2 gg = gz[yp * T + x];
-                    const float2 e = fma2(fma2(qa, d1, ql), d1, qk);
-                    const float2 vis = make_float2(exp2f(e.x), exp2f(e.y));
-                    const bool ka = !(e.x > 0.f || e.x < e_min);
-                    const bool kb = !(e.y > 0.f || e.y < e_min);
-                    // Select after the product: a skipped sample may have vis = inf (e > 0).
-                    const float2 gvr = mul2(gg, vis);
-                    const float2 gv = make_float2(ka ? gvr.x : 0.f, kb ? gvr.y : 0.f);
-                    a3 = add2(a3, gv);
-                    const float2 gvd = mul2(gv, d1);
-                    a1 = add2(a1, gvd);
-                    a2 = fma2(gvd, d1, a2);
-                    d1 = add2(d1, one);
-                }
-                z0 = add2(z0, a3);
-                z1 = add2(z1, a1);
-                r11 = add2(r11, a2);
-                const float2 gd2 = mul2(d2, a3);
-                z2 = add2(z2, gd2);
-                r22 = fma2(d2, gd2, r22);
-                r12 = fma2(d2, a1, r12);
-            }
-            const float g0 = z0.x + z0.y, g1 = z1.x + z1.y, g2 = z2.x + z2.y;
-            s0 += g0;
-            s1 += g1;
-            s2 += g2;
-            s3 = fmaf(d3, g0, s3);
-            s13 = fmaf(d3, g1, s13);
-            s23 = fmaf(d3, g2, s23);
-            s33 = fmaf(d3 * d3, g0, s33);
-        }
+        const float k2 = kVar && chain_var ? 2.f * q2.w * opac : 0.f;
+        const Rec3D<float> own{q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y};
+        float adj[3], det;
+        const bool test = active && !conic_bounded(own, adj, det);
+        const LaneSums m = __any_sync(0xffffffffu, test)
+                               ? lane_walk<kVar, true>(s_g, s_u, q0, q1, q2, e_min, k2, fx, fy, fz)
+                               : lane_walk<kVar, false>(s_g, s_u, q0, q1, q2, e_min, k2, fx, fy, fz);
         if (!active) continue;
         const float nom = -opac;
-        const float S1 = nom * s1, S2 = nom * s2, S3 = nom * s3;
-        const float S11 = nom * (r11.x + r11.y), S12 = nom * (r12.x + r12.y), S13 = nom * s13;
-        const float S22 = nom * (r22.x + r22.y), S23 = nom * s23, S33 = nom * s33;
+        const float S1 = nom * m.s1, S2 = nom * m.s2, S3 = nom * m.s3;
+        const float S11 = nom * (m.r11.x + m.r11.y), S12 = nom * (m.r12.x + m.r12.y), S13 = nom * m.s13;
+        const float S22 = nom * (m.r22.x + m.r22.y), S23 = nom * m.s23, S33 = nom * m.s33;
         // The conic again (read once more rather than held through the walk).
         const float4 c4 = __ldg(reinterpret_cast<const float4*>(rp) + 1);
         const float a = c4.x, p = c4.y, q = c4.z, bb = c4.w, rr = __ldg(&rp->c12), c = __ldg(&rp->c22);
         const float4 o0 = make_float4(-(a * S1 + p * S2 + q * S3), -(bb * S2 + p * S1 + rr * S3),
-                                      -(c * S3 + q * S1 + rr * S2), s0);
+                                      -(c * S3 + q * S1 + rr * S2), m.s0);
         const float4 o1 = make_float4(0.5f * S11, S12, S13, 0.5f * S22);
-        const float4 o2 = make_float4(S23, 0.5f * S33, 0.f, 0.f);
+        const float4 o2 = make_float4(S23, 0.5f * S33, 0.f, kVar ? opac * opac * (m.ru.x + m.ru.y) : 0.f);
         if (!kBulk && sl.slots == nullptr) {
             float* out = reinterpret_cast<float*>(grads + gid);
             red_add_v4(out, o0.x, o0.y, o0.z, o0.w);
@@ -1812,11 +1856,11 @@ template <typename S, bool kBeta, bool kVar, bool kBulk>
 int launch_vbwd_p(const VoxelGeom& g, const Rec3D<S>* rec, bool chain_var, const int32_t* offsets,
                   const int32_t* ids, const S* v_vol, const S* v_vol_var, Rec3D<S>* grads, cudaStream_t stream,
                   const VoxelSlots<S>& sl) {
-    if constexpr (std::is_same<S, float>::value && !kBeta && !kVar) {
+    if constexpr (std::is_same<S, float>::value && !kBeta) {
         if (g.T == 8) {
             const unsigned grid = g.tiles_x * g.tiles_y * g.tiles_z;
-            voxel_bwd_lanes_kernel<kBulk><<<grid, kVoxLaneThreads, 0, stream>>>(rec, offsets, ids, g, v_vol, grads,
-                                                                                  sl);
+            voxel_bwd_lanes_kernel<kVar, kBulk><<<grid, kVoxLaneThreads, 0, stream>>>(
+                rec, chain_var, offsets, ids, g, v_vol, v_vol_var, grads, sl);
             return check_launch("voxelize_to_voxels_bwd");
         }
     }
