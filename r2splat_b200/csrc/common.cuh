@@ -231,6 +231,23 @@ __device__ __forceinline__ void warp_sum8_pairs(const S (&v)[8], S& out0, S& out
     out1 = u[1];
 }
 
+// Ascending sort of one 32-bit key per lane across the warp (bitonic network,
+// 15 compare-exchange stages through shuffles); keys must be distinct.
+__device__ __forceinline__ uint32_t warp_sort_ascending(uint32_t key) {
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+    for (uint32_t k = 2u; k <= 32u; k <<= 1) {
+#pragma unroll
+        for (uint32_t j = k >> 1; j > 0u; j >>= 1) {
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, key, j);
+            const bool ascending = (lane & k) == 0u;
+            const bool lower = (lane & j) == 0u;
+            key = lower == ascending ? min(key, other) : max(key, other);
+        }
+    }
+    return key;
+}
+
 // Packed FP32x2 arithmetic (sm_100 FADD2 / FMUL2 / FFMA2): one instruction
 // evaluates two independent samples, each component rounded like the scalar
 // operation (round to nearest even).

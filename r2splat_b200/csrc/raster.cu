@@ -1085,23 +1085,6 @@ struct alignas(16) RecordStage {
     float e_min;
 };
 
-// Ascending sort of one 32-bit key per lane across the warp (bitonic network,
-// 15 compare-exchange stages through shuffles); keys must be distinct.
-__device__ __forceinline__ uint32_t warp_sort_ascending(uint32_t key) {
-    const uint32_t lane = threadIdx.x & 31u;
-#pragma unroll
-    for (uint32_t k = 2u; k <= 32u; k <<= 1) {
-#pragma unroll
-        for (uint32_t j = k >> 1; j > 0u; j >>= 1) {
-            const uint32_t other = __shfl_xor_sync(0xffffffffu, key, j);
-            const bool ascending = (lane & k) == 0u;
-            const bool lower = (lane & j) == 0u;
-            key = lower == ascending ? min(key, other) : max(key, other);
-        }
-    }
-    return key;
-}
-
 // Walks the staged records at sorted positions [p, p_end) in groups of
 // 32 / kLanes, one record per kLanes-lane group of the warp (a group without
 // a record walks nothing and stores nothing), with the packed walk

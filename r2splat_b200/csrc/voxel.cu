@@ -57,7 +57,7 @@ static __device__ unsigned int g_bulk_wait_faults;
 // sorted intersection i, flatten_ids unused), and each batch is staged by one
 // bulk copy; otherwise records are gathered through flatten_ids by cp.async.
 template <typename S, bool kBeta, bool kVar, int PPT, bool kBulk>
-__global__ void __launch_bounds__(256) voxel_fwd_kernel(const Rec3D<S>* __restrict__ records,
+__global__ void __launch_bounds__(256, 1) voxel_fwd_kernel(const Rec3D<S>* __restrict__ records,
                                                         const int32_t* __restrict__ offsets,
                                                         const int32_t* __restrict__ flatten_ids, VoxelGeom g,
                                                         S* __restrict__ volume, S* __restrict__ volume_var) {
@@ -263,12 +263,12 @@ struct alignas(16) VoxelBox {
     uint32_t origin, extent, magic_h, unused;
 };
 
-// Whether the conic Q is positive definite with tr(Q)^3 / det(Q) <= 700; then
+// Whether the conic Q is positive definite with tr(Q)^3 / det(Q) <= limit; at 700
 // the rounded sigma of any sample is within 5e-4 of sigma relative (see
 // voxel_box_bounds), and so never negative. Also gives adj(Q)'s diagonal and
 // det(Q).
 template <typename S>
-__device__ __forceinline__ bool conic_bounded(const Rec3D<S>& r, S* adj, S& det) {
+__device__ __forceinline__ bool conic_bounded(const Rec3D<S>& r, S* adj, S& det, S limit = S(700)) {
     const S a = r.c00, p = r.c01, q = r.c02, bb = r.c11, rr = r.c12, c = r.c22;
     adj[0] = bb * c - rr * rr;
     adj[1] = a * c - q * q;
@@ -276,7 +276,7 @@ __device__ __forceinline__ bool conic_bounded(const Rec3D<S>& r, S* adj, S& det)
     det = a * adj[0] - p * (p * c - rr * q) + q * (p * rr - bb * q);
     const S tr = a + bb + c;
     return a > S(0) && bb > S(0) && c > S(0) && adj[0] > S(0) && adj[1] > S(0) && adj[2] > S(0) && det > S(0) &&
-           tr * tr * tr <= S(700) * det;
+           tr * tr * tr <= limit * det;
 }
 
 // Conservative box of the voxels whose sample can pass the contribution test
@@ -289,7 +289,12 @@ __device__ __forceinline__ bool conic_bounded(const Rec3D<S>& r, S* adj, S& det)
 // half-widths sqrt(2 s' adj(Q)_ii / det(Q)). Beta: d^T Q d < 1, so d^T Q d <
 // 1.001. Half-widths are widened by 0.1 % + 0.01 voxel and by 1e-6 of the
 // coordinates' magnitude; any other case takes the whole tile.
-template <typename S, bool kBeta>
+// With kWide, Beta conics up to tr(Q)^3 / det(Q) = 5e4 (needles of 1:79) are
+// bounded too: tr / lambda_min <= tr^3 / det, so the rounded d^T Q d is within
+// 10 * 2^-24 * 5e4 = 3 % of its value, and the rounding of det (3 * 2^-24) and
+// of adj_ii >= det / tr (1.5 * 2^-24), likewise times 5e4, adds 1.4 %:
+// d^T Q d < 1.06 covers the three.
+template <typename S, bool kBeta, bool kWide = false>
 __device__ __forceinline__ bool voxel_box_bounds(const Rec3D<S>& r, uint32_t ox, uint32_t oy, uint32_t oz,
                                                  uint32_t vx, uint32_t vy, uint32_t vz, uint32_t* lo,
                                                  uint32_t* hi) {
@@ -300,6 +305,10 @@ __device__ __forceinline__ bool voxel_box_bounds(const Rec3D<S>& r, uint32_t ox,
     S adj[3], det;
     bool bounded = conic_bounded(r, adj, det);
     S reach = S(1.001);
+    if (kWide && kBeta && !bounded) {
+        bounded = conic_bounded(r, adj, det, S(5e4));
+        reach = S(1.06);
+    }
     if (!kBeta) {
         S s = log(fabs(r.o)) + S(13.815510557964274);  // ln(1e6)
         s = s + S(1e-3) * fabs(s) + S(1e-3);
@@ -340,17 +349,12 @@ __device__ __forceinline__ VoxelBox voxel_box(const Rec3D<S>& r, uint32_t ox, ui
     return box;
 }
 
-// Whether no voxel centre of the box [lo, hi] passes the contribution test of a
-// record with a bounded conic, decided conservatively. A passing voxel has
-// sigma <= s' (see voxel_box_bounds). sigma is convex, so it lies above its
-// tangent plane at any point; at the box's point nearest the centre, whose
-// offset is e, the plane's least value over the box is
-// sigma(e) + sum_i min(g_i (lo_i - p_i), g_i (hi_i - p_i)), g = Q e. The
-// margin covers the rounding of g and sigma(e).
-__device__ __forceinline__ bool misses_tile(const Rec3D<float>& r, const float* lo, const float* hi) {
-    if (fabsf(r.o) < 0.999e-6f) return true;  // sigma is not negative
-    float s = logf(fabsf(r.o)) + 13.815510557964274f;  // ln(1e6)
-    s = s + 1e-3f * fabsf(s) + 1e-3f;
+// A lower bound of sigma = d^T Q d / 2 over the box [lo, hi], for Q positive
+// definite. sigma is convex, so it lies above its tangent plane at any point;
+// at the box's point nearest the centre, whose offset is e, the plane's least
+// value over the box is sigma(e) + sum_i min(g_i (lo_i - p_i), g_i (hi_i - p_i)),
+// g = Q e. The margin covers the rounding of g and sigma(e).
+__device__ __forceinline__ float least_sigma(const Rec3D<float>& r, const float* lo, const float* hi) {
     const float px = fminf(fmaxf(r.x, lo[0]), hi[0]), py = fminf(fmaxf(r.y, lo[1]), hi[1]);
     const float pz = fminf(fmaxf(r.z, lo[2]), hi[2]);
     const float ex = px - r.x, ey = py - r.y, ez = pz - r.z;
@@ -360,8 +364,148 @@ __device__ __forceinline__ bool misses_tile(const Rec3D<float>& r, const float* 
     const float least = se + fminf(gx * (lo[0] - px), gx * (hi[0] - px)) + fminf(gy * (lo[1] - py), gy * (hi[1] - py)) +
                         fminf(gz * (lo[2] - pz), gz * (hi[2] - pz));
     const float reach = fabsf(ex) + fabsf(ey) + fabsf(ez) + (hi[0] - lo[0]) + (hi[1] - lo[1]) + (hi[2] - lo[2]);
-    const float margin = 1e-5f * (r.c00 + r.c11 + r.c22) * (fabsf(ex) + fabsf(ey) + fabsf(ez)) * reach;
-    return least - margin > s;  // false for a NaN
+    return least - 1e-5f * (r.c00 + r.c11 + r.c22) * (fabsf(ex) + fabsf(ey) + fabsf(ez)) * reach;
+}
+
+// Whether no voxel centre of the box [lo, hi] passes the contribution test of a
+// Gaussian record with a bounded conic, decided conservatively: a passing voxel
+// has sigma <= s' (see voxel_box_bounds).
+__device__ __forceinline__ bool misses_tile(const Rec3D<float>& r, const float* lo, const float* hi) {
+    if (fabsf(r.o) < 0.999e-6f) return true;  // sigma is not negative
+    float s = logf(fabsf(r.o)) + 13.815510557964274f;  // ln(1e6)
+    s = s + 1e-3f * fabsf(s) + 1e-3f;
+    return least_sigma(r, lo, hi) > s;  // false for a NaN
+}
+
+// A record's box on one 8^3 tile as the box walks read it: the first voxel's
+// centre, its index (z * 8 + y) * 8 + x in the tile, the extents and the
+// division constants (k * magic) >> 16 == k / extent.
+struct alignas(16) BoxWalk {
+    float bx, by, bz;
+    uint32_t first, w, h, area, magic_w, magic_h, rows, slot, id;
+};
+
+template <bool kWide>
+__device__ __forceinline__ BoxWalk box_walk(const Rec3D<float>& r, uint32_t ox, uint32_t oy, uint32_t oz, uint32_t vx,
+                                            uint32_t vy, uint32_t vz) {
+    uint32_t lo[3], hi[3];
+    BoxWalk b{};
+    if (!voxel_box_bounds<float, true, kWide>(r, ox, oy, oz, vx, vy, vz, lo, hi)) return b;
+    // A needle across the tile grid reaches few of the tiles that its bounding box covers.
+    const float first[3] = {ox + 0.5f, oy + 0.5f, oz + 0.5f};
+    const float last[3] = {first[0] + float(vx - 1u), first[1] + float(vy - 1u), first[2] + float(vz - 1u)};
+    float adj[3], det;
+    if (conic_bounded(r, adj, det, 5e4f) && least_sigma(r, first, last) > 0.53f) return b;  // d^T Q d > 1.06
+    b.bx = static_cast<float>(ox + lo[0]) + 0.5f;
+    b.by = static_cast<float>(oy + lo[1]) + 0.5f;
+    b.bz = static_cast<float>(oz + lo[2]) + 0.5f;
+    b.first = (lo[2] * 8u + lo[1]) * 8u + lo[0];
+    b.w = hi[0] - lo[0] + 1u;
+    b.h = hi[1] - lo[1] + 1u;
+    b.rows = b.h * (hi[2] - lo[2] + 1u);
+    b.area = b.w * b.rows;
+    b.magic_w = (65536u + b.w - 1u) / b.w;
+    b.magic_h = (65536u + b.h - 1u) / b.h;
+    return b;
+}
+
+// fp32 Beta forward at T = 8, one warp per tile: a Beta record reaches a few
+// voxels of a tile (13 % at ordinary scales), so the lanes walk the voxels of
+// its box, a lane a voxel, and the tile's sums stay in shared memory. The
+// records are taken one after the other, so a voxel's samples are added in
+// list order, each with the expression and rounding of voxel_fwd_kernel; a
+// voxel outside the box fails the support test there. Bound by the issue of a
+// record's two or three steps (some 130 instructions) and their latency.
+// 100,000 primitives in 192^3 (0.44 M pairs): 0.172 -> 0.057 ms; 500,000 with
+// the variance in 384^3 (5.3 M): 1.97 -> 0.99 ms (every voxel of the tile
+// evaluated before). A needle's box can be the whole tile, which costs what it
+// did.
+constexpr int kVoxBetaWarps = 2;
+// Grids of at most three tiles per SM keep the forms with several warps a tile (216 tiles: 0.019 / 0.021 ms forward,
+// 0.020 / 0.025 VJP; 512 tiles 0.025 / 0.023 and 0.027 / 0.027; 1,728 tiles 0.060 / 0.025 and 0.056 / 0.031).
+constexpr uint32_t kVoxBetaTiles = 444;
+
+template <bool kVar, bool kBulk>
+__global__ void __launch_bounds__(32 * kVoxBetaWarps) voxel_beta_fwd_kernel(
+    const Rec3D<float>* __restrict__ records, const int32_t* __restrict__ offsets,
+    const int32_t* __restrict__ flatten_ids, VoxelGeom g, float* __restrict__ volume, float* __restrict__ volume_var) {
+    constexpr uint32_t T = 8u;
+    __shared__ float s_accs[kVoxBetaWarps][T * T * T];
+    __shared__ float s_accvs[kVoxBetaWarps][kVar ? T * T * T : 1];
+    __shared__ Rec3D<float> s_recs[kVoxBetaWarps][32];
+    __shared__ BoxWalk s_boxes[kVoxBetaWarps][32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t n_tiles = g.tiles_x * g.tiles_y * g.tiles_z;
+    const uint32_t key = blockIdx.x * kVoxBetaWarps + warp;
+    if (key >= n_tiles) return;
+    float* s_acc = s_accs[warp];
+    float* s_accv = s_accvs[warp];
+    Rec3D<float>* s_rec = s_recs[warp];
+    BoxWalk* s_box = s_boxes[warp];
+    const uint32_t tz = key / (g.tiles_x * g.tiles_y);
+    const uint32_t rem = key - tz * g.tiles_x * g.tiles_y;
+    const uint32_t ty = rem / g.tiles_x, tx = rem - ty * g.tiles_x;
+    const uint32_t ox = tx * T, oy = ty * T, oz = tz * T;
+    if (ox >= g.dim2 || oy >= g.dim1 || oz >= g.dim0) return;
+    const uint32_t vx = min(T, g.dim2 - ox), vy = min(T, g.dim1 - oy), vz = min(T, g.dim0 - oz);
+    const int32_t start = offsets[key];
+    const int32_t n_total = g.n_dev != nullptr ? int32_t(*g.n_dev) : int32_t(g.n_isects);
+    const int32_t end = (key + 1 == n_tiles) ? n_total : offsets[key + 1];
+#pragma unroll
+    for (uint32_t i = 0; i < T * T * T; i += 32u) {
+        s_acc[i + lane] = 0.f;
+        if (kVar) s_accv[i + lane] = 0.f;
+    }
+    for (int32_t b = start; b < end; b += 32) {
+        const int32_t idx = b + int32_t(lane);
+        uint32_t area = 0u;
+        __syncwarp();  // the previous batch has been read
+        if (idx < end) {
+            const Rec3D<float> r = records[kBulk ? idx : flatten_ids[idx]];
+            const BoxWalk box = box_walk<true>(r, ox, oy, oz, vx, vy, vz);
+            area = box.area;
+            s_rec[lane] = r;
+            s_box[lane] = box;
+        }
+        uint32_t live = __ballot_sync(0xffffffffu, area != 0u);
+        __syncwarp();
+        while (live != 0u) {
+            const uint32_t s = __ffs(int(live)) - 1u;
+            live &= live - 1u;
+            const Rec3D<float> r = s_rec[s];
+            const BoxWalk box = s_box[s];
+            for (uint32_t k = lane; k < box.area; k += 32u) {
+                const uint32_t row = (k * box.magic_w) >> 16, x = k - row * box.w;
+                const uint32_t z = (row * box.magic_h) >> 16, y = row - z * box.h;
+                const uint32_t at = box.first + (z * T + y) * T + x;
+                const float d1 = r.x - (box.bx + static_cast<float>(x)), d2 = r.y - (box.by + static_cast<float>(y));
+                const float d3 = r.z - (box.bz + static_cast<float>(z));
+                const float sq = fmaf(__fmul_rn(r.c22, d3), d3,
+                                      fmaf(__fmul_rn(r.c00, d1), d1, __fmul_rn(__fmul_rn(r.c11, d2), d2)));
+                const float qf = fmaf(__fmul_rn(__fmul_rn(2.f, r.c12), d2), d3,
+                                      fmaf(__fmul_rn(__fmul_rn(2.f, r.c02), d1), d3,
+                                           fmaf(__fmul_rn(__fmul_rn(2.f, r.c01), d1), d2, sq)));
+                if (!(qf < 0.f || qf >= 1.f)) {
+                    const float alpha = r.o * pow(1.f - qf, r.beta);
+                    if (!(fabsf(alpha) < 1e-5f)) {
+                        s_acc[at] += alpha;
+                        if (kVar) s_accv[at] = fmaf(__fmul_rn(r.q, alpha), alpha, s_accv[at]);
+                    }
+                }
+            }
+            __syncwarp();  // the next record's lanes add to the same voxels
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (uint32_t i = 0; i < T * T * T; i += 32u) {
+        const uint32_t at = i + lane, x = at & 7u, y = (at >> 3) & 7u, z = at >> 6;
+        if (x < vx && y < vy && z < vz) {
+            const size_t vid = (size_t(oz + z) * g.dim1 + (oy + y)) * g.dim2 + (ox + x);
+            volume[vid] = s_acc[at];
+            if (kVar) volume_var[vid] = s_accv[at];
+        }
+    }
 }
 
 // fp32 Gaussian forward at T = 8, one warp per tile: a lane owns 4 x 2 x 2
@@ -1334,6 +1478,230 @@ __global__ void __launch_bounds__(kVoxLaneThreads, 4) voxel_bwd_lanes_kernel(
     }
 }
 
+// Tile VJP of fp32 Beta records on 8^3 tiles, one warp per tile and eight lanes
+// per (tile, primitive) pair, four pairs of about equal boxes at a time: a lane
+// walks every eighth row of the record's box (about 25 rows of five voxels),
+// and one exchange of 12 sums over the eight lanes ends a pair. Every sum is
+// formed as in voxel_bwd_kernel, down to the rounding and the order, and the 12
+// values written are the same bit for bit: near the edge of the support of a
+// Beta with an exponent below one a sample's weight is as large as its distance
+// to the edge is small, so sums in another order differ by more than rounding
+// usually does.
+// A warp a tile, because tiles hold few Beta pairs (48 in the larger of the
+// scenes below) and a block of eight warps waited on its staging for them.
+// Kernel and slot sum, 100,000 primitives in 192^3: 0.238 -> 0.120 ms; 500,000
+// with the variance in 384^3: 3.07 -> 2.31 ms. 10 blocks a SM (96 registers)
+// against 12 with spills and 8: 2.31 / 2.46 / 2.45 ms. (A lane per voxel of the
+// box takes 1.82 ms in the second scene, with sums in another order.)
+template <bool kVar, bool kBulk>
+__global__ void __launch_bounds__(32 * kVoxBetaWarps, 10) voxel_beta_bwd_kernel(
+    const Rec3D<float>* __restrict__ records, bool chain_var, const int32_t* __restrict__ offsets,
+    const int32_t* __restrict__ flatten_ids, VoxelGeom g, const float* __restrict__ v_volume,
+    const float* __restrict__ v_volume_var, Rec3D<float>* __restrict__ grads, VoxelSlots<float> sl) {
+    constexpr uint32_t T = 8u;
+    __shared__ float s_gs[kVoxBetaWarps][T * T * T];
+    __shared__ float s_us[kVoxBetaWarps][kVar ? T * T * T : 1];
+    __shared__ Rec3D<float> s_recs[kVoxBetaWarps][32];
+    __shared__ BoxWalk s_boxes[kVoxBetaWarps][32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t n_tiles = g.tiles_x * g.tiles_y * g.tiles_z;
+    const uint32_t key = blockIdx.x * kVoxBetaWarps + warp;
+    if (key >= n_tiles) return;
+    float* s_g = s_gs[warp];
+    float* s_u = s_us[warp];
+    Rec3D<float>* s_rec = s_recs[warp];
+    BoxWalk* s_box = s_boxes[warp];
+    const uint32_t tz = key / (g.tiles_x * g.tiles_y);
+    const uint32_t rem = key - tz * g.tiles_x * g.tiles_y;
+    const uint32_t ty = rem / g.tiles_x, tx = rem - ty * g.tiles_x;
+    const uint32_t ox = tx * T, oy = ty * T, oz = tz * T;
+    if (ox >= g.dim2 || oy >= g.dim1 || oz >= g.dim0) return;
+    const uint32_t vx = min(T, g.dim2 - ox), vy = min(T, g.dim1 - oy), vz = min(T, g.dim0 - oz);
+    const int32_t start = offsets[key];
+    const int32_t n_total = g.n_dev != nullptr ? int32_t(*g.n_dev) : int32_t(g.n_isects);
+    const int32_t end = (key + 1 == n_tiles) ? n_total : offsets[key + 1];
+    if (end <= start) return;
+#pragma unroll 4
+    for (uint32_t i = 0; i < T * T * T; i += 32u) {
+        const uint32_t at = i + lane, x = at & 7u, y = (at >> 3) & 7u, z = at >> 6;
+        float gv = 0.f, uv = 0.f;
+        if (x < vx && y < vy && z < vz) {
+            const size_t vid = (size_t(oz + z) * g.dim1 + (oy + y)) * g.dim2 + (ox + x);
+            if (v_volume != nullptr) gv = v_volume[vid];
+            if (kVar) uv = v_volume_var[vid];
+        }
+        s_g[at] = gv;
+        if (kVar) s_u[at] = uv;
+    }
+    const uint32_t group = lane >> 3, sub = lane & 7u;
+    for (int32_t b = start; b < end; b += 32) {
+        const int32_t idx = b + int32_t(lane);
+        uint32_t area = 0u;
+        __syncwarp();  // the adjoints are staged; the previous batch has been read
+        if (idx < end) {
+            int32_t gid = 0;
+            uint32_t slot = 0xffffffffu;
+            Rec3D<float> r;
+            if constexpr (kBulk) {
+                r = records[idx];
+                slot = __float_as_uint(r.pad0);  // the pack kernel's slot (or 0xffffffff)
+            } else {
+                gid = flatten_ids[idx];
+                r = records[gid];
+                if (sl.slots != nullptr) {
+                    const uint64_t first = gid > 0 ? uint64_t(sl.cum[gid - 1]) : 0u;
+                    const float mv[3] = {r.x, r.y, r.z};
+                    uint32_t blo[3], bhi[3];
+                    if (tile_box_3d(mv, sl.radii + 3 * size_t(gid), T, g.tiles_x, g.tiles_y, g.tiles_z, blo, bhi)) {
+                        const uint64_t local = (uint64_t(tz - blo[2]) * (bhi[1] - blo[1]) + (ty - blo[1])) *
+                                                   (bhi[0] - blo[0]) + (tx - blo[0]);
+                        if (first + local < sl.capacity) slot = uint32_t(first + local);
+                    }
+                }
+            }
+            BoxWalk box = box_walk<false>(r, ox, oy, oz, vx, vy, vz);
+            area = box.area;
+            box.slot = slot;
+            box.id = uint32_t(gid);
+            s_rec[lane] = r;
+            s_box[lane] = box;
+            if (area == 0u && slot != 0xffffffffu) {
+                float4* out = reinterpret_cast<float4*>(sl.slots + size_t(slot) * 12u);
+                out[0] = out[1] = out[2] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+        const uint32_t n_live = __popc(__ballot_sync(0xffffffffu, area != 0u));
+        // Boxes in order of size, so the four pairs of a step take about the same number of steps.
+        const uint32_t sorted = warp_sort_ascending(area != 0u ? (area << 5) | lane : 0xffffffe0u | lane);
+        __syncwarp();
+        for (uint32_t p = 0; p < n_live; p += 4u) {
+            const bool active = p + group < n_live;  // a group without a pair follows the last one and writes nothing
+            const uint32_t at_rec = __shfl_sync(0xffffffffu, sorted, min(p + group, n_live - 1u)) & 31u;
+            const Rec3D<float> r = s_rec[at_rec];
+            const BoxWalk box = s_box[at_rec];
+            const uint32_t rows = active ? box.rows : 0u;
+            uint32_t row_end = box.rows, x_end = box.w;  // the step's largest box in each direction
+#pragma unroll
+            for (int offset = 8; offset < 32; offset <<= 1) {
+                row_end = max(row_end, __shfl_xor_sync(0xffffffffu, row_end, offset));
+                x_end = max(x_end, __shfl_xor_sync(0xffffffffu, x_end, offset));
+            }
+            const float a = r.c00, pp = r.c01, q = r.c02, bb = r.c11, rr = r.c12, c = r.c22;
+            const float uq = chain_var ? r.q : 0.f;
+            // Lane `sub` takes rows sub + 8 i (and 32 on) and adds their sums in voxel_bwd_kernel's order, in which a lane
+            // l takes rows l and l + 32 and the lanes are combined by halves: (0 + 2) + (1 + 3) over i, then the lanes.
+            float part[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) part[i] = 0.f;
+            for (uint32_t half = 0; half < 2u && 8u * half < row_end; ++half) {
+                float sum[12];
+#pragma unroll
+                for (int i = 0; i < 12; ++i) sum[i] = 0.f;
+                for (uint32_t quarter = half; quarter < 4u && 8u * quarter < row_end; quarter += 2u) {
+                    float P[12];
+#pragma unroll
+                    for (int i = 0; i < 12; ++i) P[i] = 0.f;
+                    for (uint32_t row = 8u * quarter + sub, r0 = 8u * quarter; r0 < row_end; row += 32u, r0 += 32u) {
+                        const bool row_valid = row < rows;
+                        const uint32_t zz = row_valid ? (row * box.magic_h) >> 16 : 0u;
+                        const uint32_t yy = row_valid ? row - zz * box.h : 0u;
+                        const uint32_t at = box.first + (zz * T + yy) * T;
+                        const float py = box.by + static_cast<float>(yy), pz = box.bz + static_cast<float>(zz);
+                        const float d2 = r.y - py, d3 = r.z - pz;
+                        // The contraction voxel_bwd_kernel's expressions get, spelled out.
+                        const float K = fmaf(__fmul_rn(2.f * rr, d2), d3,
+                                             fmaf(__fmul_rn(c, d3), d3, __fmul_rn(__fmul_rn(bb, d2), d2)));
+                        const float L = 2.f * fmaf(q, d3, __fmul_rn(pp, d2));
+                        float A0 = 0.f, A1 = 0.f, A2 = 0.f, A3 = 0.f, A4 = 0.f, A5 = 0.f;
+                        float px = box.bx;
+                        const uint32_t width = row_valid ? box.w : 0u;
+#pragma unroll 2
+                        for (uint32_t i = 0; i < x_end; ++i, px += 1.f) {
+                            const bool valid = i < width;
+                            float v = valid ? s_g[at + i] : 0.f;
+                            const float vv = (kVar && valid) ? s_u[at + i] : 0.f;
+                            const float d1 = r.x - px;
+                            const float qf = __fadd_rn(fmaf(L, d1, __fmul_rn(__fmul_rn(a, d1), d1)), K);
+                            const float h_raw = __fadd_rn(1.f, -qf);
+                            const bool in_support = valid && !(qf < 0.f || h_raw <= 0.f);
+                            const float hh = in_support ? h_raw : 1.f;  // keeps the logarithm finite on skipped samples
+                            const float lg = log2f(hh);
+                            const float vis_raw = exp2f(r.beta * lg);
+                            const float alpha_raw = r.o * vis_raw;
+                            const bool keep = in_support && !(fabsf(alpha_raw) < 1e-5f);
+                            const float vis = keep ? vis_raw : 0.f;
+                            const float alpha = keep ? alpha_raw : 0.f;
+                            v = keep ? v : 0.f;
+                            if (kVar) {
+                                A4 = fmaf(__fmul_rn(vv, alpha), alpha, A4);
+                                v = fmaf(__fmul_rn(2.f * uq, alpha), vv, v);
+                            }
+                            const float wgt = __fmul_rn(__fmul_rn(-r.o * r.beta, vis_raw / hh), v);
+                            A3 = fmaf(v, vis, A3);
+                            A5 = fmaf(__fmul_rn(v, alpha), lg * 0.6931471805599453f, A5);  // ln hh = ln 2 log2 hh
+                            const float wd = __fmul_rn(wgt, d1);
+                            A0 += wgt;
+                            A1 += wd;
+                            A2 = fmaf(wd, d1, A2);
+                        }
+                        P[0] += A1;
+                        P[1] = fmaf(d2, A0, P[1]);
+                        P[2] = fmaf(d3, A0, P[2]);
+                        P[3] += A3;
+                        P[4] += A2;
+                        P[5] = fmaf(d2, A1, P[5]);
+                        P[6] = fmaf(d3, A1, P[6]);
+                        P[7] = fmaf(__fmul_rn(d2, d2), A0, P[7]);
+                        P[8] = fmaf(__fmul_rn(d2, d3), A0, P[8]);
+                        P[9] = fmaf(__fmul_rn(d3, d3), A0, P[9]);
+                        P[10] += A5;
+                        P[11] += A4;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 12; ++i) sum[i] += P[i];
+                }
+#pragma unroll
+                for (int i = 0; i < 12; ++i) part[i] += sum[i];
+            }
+            // Exchange of halves over the eight lanes: lane `sub` ends with sums 2 sub and 2 sub + 1.
+            float w8[8], w4[4], lo, hi;
+            const bool up4 = (sub & 4u) != 0u, up2 = (sub & 2u) != 0u, up1 = (sub & 1u) != 0u;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                w8[i] = (up4 ? part[i + 8] : part[i]) + __shfl_xor_sync(0xffffffffu, up4 ? part[i] : part[i + 8], 4);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                w4[i] = (up2 ? w8[i + 4] : w8[i]) + __shfl_xor_sync(0xffffffffu, up2 ? w8[i] : w8[i + 4], 2);
+            lo = (up1 ? w4[2] : w4[0]) + __shfl_xor_sync(0xffffffffu, up1 ? w4[0] : w4[2], 1);
+            hi = (up1 ? w4[3] : w4[1]) + __shfl_xor_sync(0xffffffffu, up1 ? w4[1] : w4[3], 1);
+            // Lanes 0 and 1 hold (S1, S2) and (S3, Svis): x, y, z need all three first moments.
+            const float S1 = __shfl_sync(0xffffffffu, lo, 0, 8), S2 = __shfl_sync(0xffffffffu, hi, 0, 8);
+            const float S3 = __shfl_sync(0xffffffffu, lo, 1, 8);
+            if (sub == 0u) {
+                lo = 2.f * fmaf(q, S3, fmaf(a, S1, __fmul_rn(pp, S2)));
+                hi = 2.f * fmaf(rr, S3, fmaf(bb, S2, __fmul_rn(pp, S1)));
+            } else if (sub == 1u) {
+                lo = 2.f * fmaf(rr, S2, fmaf(c, S3, __fmul_rn(q, S1)));
+            } else if (sub == 2u) {
+                hi *= 2.f;  // c01
+            } else if (sub == 3u) {
+                lo *= 2.f;  // c02
+            } else if (sub == 4u) {
+                lo *= 2.f;  // c12
+            }
+            if (active && sub < 6u) {
+                if (!kBulk && sl.slots == nullptr) {
+                    float* out = reinterpret_cast<float*>(grads + box.id) + 2u * sub;
+                    atomicAdd(out, lo);
+                    atomicAdd(out + 1, hi);
+                } else if (box.slot != 0xffffffffu) {
+                    *reinterpret_cast<float2*>(sl.slots + size_t(box.slot) * 12u + 2u * sub) = make_float2(lo, hi);
+                }
+            }
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Record-parallel voxel VJP (the explicit path).
 //
@@ -1828,6 +2196,14 @@ int launch_vfwd_p(const VoxelGeom& g, const Rec3D<S>* rec, const int32_t* offset
             return check_launch("voxelize_to_voxels_fwd");
         }
     }
+    if constexpr (kBeta && std::is_same<S, float>::value) {
+        if (g.T == 8 && g.tiles_x * g.tiles_y * g.tiles_z > kVoxBetaTiles) {
+            voxel_beta_fwd_kernel<kVar, kBulk>
+                <<<blocks_for(g.tiles_x * g.tiles_y * g.tiles_z, kVoxBetaWarps), 32 * kVoxBetaWarps, 0, stream>>>(
+                    rec, offsets, ids, g, vol, vol_var);
+            return check_launch("voxelize_to_voxels_fwd");
+        }
+    }
     // Four consecutive voxels of a row per thread: T^2 rows of ceil(T / 4) segments.
     const unsigned nt = (g.T * g.T * ((g.T + 3) / 4) + 31) / 32 * 32;
     return launch_vfwd_t<S, kBeta, kVar, 4, kBulk>(g, rec, offsets, ids, vol, vol_var, nt, stream);
@@ -1861,6 +2237,14 @@ int launch_vbwd_p(const VoxelGeom& g, const Rec3D<S>* rec, bool chain_var, const
             const unsigned grid = g.tiles_x * g.tiles_y * g.tiles_z;
             voxel_bwd_lanes_kernel<kVar, kBulk><<<grid, kVoxLaneThreads, 0, stream>>>(
                 rec, chain_var, offsets, ids, g, v_vol, v_vol_var, grads, sl);
+            return check_launch("voxelize_to_voxels_bwd");
+        }
+    }
+    if constexpr (std::is_same<S, float>::value && kBeta) {
+        if (g.T == 8 && g.tiles_x * g.tiles_y * g.tiles_z > kVoxBetaTiles) {
+            voxel_beta_bwd_kernel<kVar, kBulk>
+                <<<blocks_for(g.tiles_x * g.tiles_y * g.tiles_z, kVoxBetaWarps), 32 * kVoxBetaWarps, 0, stream>>>(
+                    rec, chain_var, offsets, ids, g, v_vol, v_vol_var, grads, sl);
             return check_launch("voxelize_to_voxels_bwd");
         }
     }
