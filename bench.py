@@ -79,9 +79,9 @@ SOURCE_FORM_OPS = {
 # these, the lower of the two counts.
 CONTRACTED_OPS = {"raster_render": 11, "raster_render_bwd": 30, "voxel_render": 21, "voxel_render_bwd": 48}
 ACCUMULATE_KERNELS = {
-    "raster_render": "raster_fwd_pair_kernel (tile forward, two pixels per lane)",
+    "raster_render": "raster_fwd_group_kernel (tile forward, a hit list per 4x4 pixel block)",
     "raster_render_bwd": "raster_record_bwd_kernel (record-parallel raster VJP)",
-    "voxel_render": "voxel_fwd_kernel (tile forward, two rows of eight voxels per thread, bulk-staged packed records)",
+    "voxel_render": "voxel_fwd_block_kernel (tile forward, 4 x 2 x 2 voxels per lane, bulk-staged packed records)",
     "voxel_render_bwd": ("voxel_bwd_lanes_kernel (one lane per (tile, primitive) pair walking the 8^3 tile in "
                          "lockstep, packed records)"),
 }

@@ -1,14 +1,15 @@
 // Voxelization: per-tile (T^3 voxels) accumulation of Gaussian / Beta
 // densities at voxel centres, and its VJP, on packed per-primitive records.
 //
-// Same schedule as the rasterizer: one CTA per 3D tile, the tile's
-// intersection list gathered into shared memory with cp.async in buffered
-// batches (records are [N] x 64 B and stay in L2). Forward threads own a 4 x 2 x
-// 2 block (Gaussian fp32 at T = 8), 4 voxels of a row, or single voxels;
-// backward warps own one record at a time over the record's box in the tile,
-// warp-reduce, and either write the record's partial adjoints to its own slot
-// (reduced per primitive in a fixed order afterwards) or add them with vector
-// atomics.
+// The tiles' intersection lists are taken in buffered batches (records are [N] x
+// 64 B and stay in L2, or are packed per tile in list order). Forward: a warp
+// per tile with 4 x 2 x 2 voxels a lane (Gaussian fp32 at T = 8) or lanes on a
+// record's box (Beta fp32 at T = 8), else a block per tile with 4 voxels of a
+// row or single voxels a thread. Backward at T = 8 in fp32: a lane per (tile,
+// primitive) pair (Gaussian) or eight lanes on its box's rows (Beta), else a
+// warp per pair over the record's box in the tile. A pair's partial adjoints go
+// to its own slot (reduced per primitive in a fixed order afterwards) or are
+// added with atomics.
 //
 // Per-sample arithmetic keeps the reference's expression forms
 // (VoxelizeToVoxelsFwd.cu:180-215, :555-580; VoxelizeToVoxelsBwd.cu:397-433,
