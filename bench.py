@@ -81,9 +81,9 @@ CONTRACTED_OPS = {"raster_render": 11, "raster_render_bwd": 30, "voxel_render": 
 ACCUMULATE_KERNELS = {
     "raster_render": "raster_fwd_group_kernel (tile forward, a hit list per 4x4 pixel block)",
     "raster_render_bwd": "raster_record_bwd_kernel (record-parallel raster VJP)",
-    "voxel_render": "voxel_fwd_block_kernel (tile forward, 4 x 2 x 2 voxels per lane, bulk-staged packed records)",
+    "voxel_render": "voxel_fwd_block_kernel (tile forward, 4 x 2 x 2 voxels per lane)",
     "voxel_render_bwd": ("voxel_bwd_lanes_kernel (one lane per (tile, primitive) pair walking the 8^3 tile in "
-                         "lockstep, packed records)"),
+                         "lockstep)"),
 }
 # FP32 operations per sample of the Beta raster VJP with the variance branch in the reference's form
 # (RasterizeToPixelsBwd.cu:817-1046), counted by the same rule: offsets 2, d^2 9, h 1, pow argument 1,

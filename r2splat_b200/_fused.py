@@ -48,6 +48,8 @@ VOXEL_SLOT_BUDGET_BYTES = 8 << 30
 # that copy and the VJP's slots fit this budget together; otherwise the tile kernels gather the records
 # through the lists, as the reference's do.
 VOXEL_PACK_BUDGET_BYTES = VOXEL_SLOT_BUDGET_BYTES
+# The same for fp32 Gaussians on 8^3 tiles, see voxel_packs.
+VOXEL_GAUSSIAN_PACK_BYTES = 16 << 20
 
 
 def _ptr(t: Optional[Tensor]):
@@ -491,6 +493,22 @@ def pack_tile_records(records, offsets, flatten_ids, radii, tile_cum, m, shape, 
     return packed
 
 
+def voxel_packs(dtype, beta: bool, tile_size, m) -> bool:
+    """Whether the voxel forward copies its m intersections' records into list order.
+
+    The copy costs a pass that writes 64 bytes an intersection, and saves the tile kernels the gather through the
+    lists. The warp-per-tile Gaussian kernels hide that gather (6.8 M intersections: pack 0.135 ms, forward 1.280 packed
+    and 1.293 gathered, VJP 1.609 and 1.656; 1.1 M with variance: 0.029, 0.298 / 0.297, 0.403 / 0.411), so they gather
+    beyond a size at which the pass is no more than its launches. The Beta VJP gains more from the slots in the records
+    (5.3 M: 0.111, 0.990 / 0.999, 2.319 / 2.464).
+    """
+    size = 4 if dtype == torch.float32 else 8
+    budget = VOXEL_PACK_BUDGET_BYTES
+    if dtype == torch.float32 and not beta and tile_size == 8:
+        budget = min(budget, VOXEL_GAUSSIAN_PACK_BYTES)
+    return m * (16 + 12) * size <= budget
+
+
 def voxel_forward(means, quats, scales, densities, shape, extent, center, beta, uncertainty, eps, radius_clip,
                   tile_size=VOXEL_TILE, before_count=None):
     device = means.device
@@ -505,7 +523,7 @@ def voxel_forward(means, quats, scales, densities, shape, extent, center, beta, 
     ty = (height + tile_size - 1) // tile_size
     tz = (depth + tile_size - 1) // tile_size
     packed = None
-    if m * (16 + 12) * means.element_size() <= VOXEL_PACK_BUDGET_BYTES:
+    if voxel_packs(means.dtype, beta is not None, tile_size, m):
         with _stage("voxel_pack"):
             packed = pack_tile_records(records, offsets, flatten_ids, radii, tile_cum, m, shape, tile_size)
     with _stage("voxel_render"):
