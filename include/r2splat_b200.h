@@ -360,7 +360,9 @@ int r2s_raster_project(int dtype, const void* means, const void* covars, const v
 int r2s_scan_tile_counts(const int32_t* counts, uint64_t n, int64_t* cum, void* workspace,
                          size_t workspace_bytes, void* stream);
 
-/* Emits the sorted 2D intersections from precomputed rectangles (no radii). */
+/* Emits the sorted 2D intersections from precomputed rectangles (no radii).
+ * n_isects: the scan's last entry, which every array is sized by; nothing is
+ * written past it, whatever the scan holds. */
 int r2s_raster_emit(const uint16_t* rects, uint32_t C, uint32_t N, uint32_t tiles_x,
                     uint32_t tiles_y, const int64_t* cum_tiles, int64_t n_isects,
                     int64_t* isect_ids, int32_t* flatten_ids, int32_t* offsets, void* workspace,

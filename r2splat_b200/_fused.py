@@ -160,7 +160,7 @@ class RasterState:
     isect_ids: Tensor
     flatten_ids: Tensor
     ratio: Optional[Tensor]
-    n_isects: int
+    n_isects: Optional[int]  # None: not counted
     width: int
     height: int
     tile_size: int = RASTER_TILE
@@ -322,18 +322,18 @@ def raster_forward(means, quats, scales, densities, viewmats, Ks, width, height,
 
 
 def raster_vjp_state(means, quats, scales, densities, viewmats, Ks, width, height, beta, eps, radius_clip,
-                     tile_size=RASTER_TILE, n_isects=0):
+                     tile_size=RASTER_TILE):
     """What the raster VJP reads (covariances, packed records, tile rectangles), rebuilt without the image.
 
-    ``n_isects`` is the forward's intersection count of the same inputs; the VJP rebuilds the tile lists from it where
-    it reads them.
+    Nothing is carried over from the forward: the inputs may have changed since (cameras written in place, saved
+    tensors that a hook stored in a narrower type), so the VJP counts the intersections anew where it lists them.
     """
     covars = _covariances(quats, scales)
     ratio = beta_path_ratio(beta) if beta is not None else None
-    records, rects, counts = _raster_project(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps,
-                                             radius_clip, tile_size)
-    return RasterState(covars, records, None, None, None, ratio, n_isects, width, height, tile_size,
-                       extra={"rects": rects, "counts": counts})
+    records, rects, _ = _raster_project(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps,
+                                        radius_clip, tile_size)
+    return RasterState(covars, records, None, None, None, ratio, None, width, height, tile_size,
+                       extra={"rects": rects})
 
 
 def voxel_vjp_state(means, quats, scales, densities, shape, extent, center, beta, uncertainty, eps, radius_clip,
@@ -349,6 +349,29 @@ def voxel_vjp_state(means, quats, scales, densities, shape, extent, center, beta
                       layer_cum, n_items)
 
 
+def _raster_vjp_lists(state: RasterState, dtype, beta: bool, variance: bool):
+    """(flatten_ids, offsets, cum, n_isects) for the tile-parallel VJP, or None where it walks the records.
+
+    Lists that the state does not hold are built from its rectangles and their own count, read here: a count from
+    elsewhere could disagree with the rectangles, and the lists' buffers are sized by it.
+    """
+    form = (dtype, beta, variance, state.tile_size, state.width, state.height)
+    if not raster_vjp_takes_tiles(*form, 0):
+        return None
+    if state.offsets is not None:
+        return ((state.flatten_ids, state.offsets, state.extra["cum"], state.n_isects)
+                if raster_vjp_takes_tiles(*form, state.n_isects) else None)
+    rects = state.extra["rects"]
+    # Rectangles are in tiles, below 2^13 on this path, so 16-bit differences are exact.
+    x0, y0, x1, y1 = rects.unbind(-1)
+    cum = _raster_scan(((x1 - x0).int() * (y1 - y0)).contiguous())
+    m = _read_total(cum)
+    if not raster_vjp_takes_tiles(*form, m):
+        return None
+    _, flatten_ids, offsets = _raster_lists(rects, cum, m, state.width, state.height, state.tile_size)
+    return flatten_ids, offsets, cum, m
+
+
 def raster_backward(state: RasterState, means, quats, scales, densities, beta, uncertainty, viewmats, Ks, eps,
                     v_image, v_variance, detach_variance):
     """Explicit projection VJP -> (v_means, v_quats, v_scales, v_densities, v_beta, v_uncertainty)."""
@@ -360,20 +383,15 @@ def raster_backward(state: RasterState, means, quats, scales, densities, beta, u
     # With the variance branch: one uncertainty adjoint per record, summed over cameras in order.
     v_unc_cn = means.new_empty((c, n)) if v_variance is not None else None
     v_unc = means.new_empty((n,)) if v_variance is not None else None
-    rects, m = state.extra["rects"], state.n_isects
-    if raster_vjp_takes_tiles(means.dtype, beta is not None, v_variance is not None, tile, state.width, state.height,
-                              m):
-        if "cum" not in state.extra:
-            state.extra["cum"] = _raster_scan(state.extra["counts"])
-        if state.offsets is None:
-            _, flatten_ids, offsets = _raster_lists(rects, state.extra["cum"], m, state.width, state.height, tile)
-        else:
-            flatten_ids, offsets = state.flatten_ids, state.offsets
+    rects = state.extra["rects"]
+    lists = _raster_vjp_lists(state, means.dtype, beta is not None, v_variance is not None)
+    if lists is not None:
+        flatten_ids, offsets, cum, m = lists
         with _stage("raster_render_bwd"):
             slots = means.new_empty((max(m, 1), RASTER_SLOT_BYTES // 4))
             _backend.call("r2s_raster_tile_bwd", _ptr(state.records), _ptr(rects), _ptr(uncertainty),
                           int(bool(detach_variance)), _ptr(offsets), _ptr(flatten_ids), m, None,
-                          _ptr(state.extra["cum"]), _ptr(v_image), _ptr(v_variance), c, n, state.width, state.height,
+                          _ptr(cum), _ptr(v_image), _ptr(v_variance), c, n, state.width, state.height,
                           tile, offsets.shape[2], offsets.shape[1], _ptr(slots), slots.shape[0], _ptr(grads),
                           _ptr(v_unc_cn), stream)
     else:

@@ -10,7 +10,8 @@ With ``recompute=True`` the forward keeps only its (validated) inputs and the
 backward rebuilds what the VJP reads:
 * rasterize: the parameter transform and the projection (packed records and
   tile rectangles), and the intersection lists where the VJP reads them (fp32
-  Gaussians with the variance branch).
+  Gaussians with the variance branch), counted anew: cameras that were written
+  since the forward give the gradients at the new cameras.
 * voxelize: the parameter transform, the voxel mapping and the scan of the
   per-primitive tile-box layer counts. The record-parallel voxel VJP walks
   each primitive's tile box, so here too the intersection lists are neither
@@ -54,7 +55,6 @@ class _Rasterize(torch.autograd.Function):
         ctx.radius_clip = _options(beta, eps, radius_clip, detach_variance)[1]
         ctx.detach_variance = detach_variance
         ctx.cameras = (context.buffers["viewmats"], context.buffers["Ks"])
-        ctx.n_isects = context.buffers["state"].n_isects if "state" in context.buffers else 0
         ctx.save_for_backward(*context.primitives)
         if recompute:
             context.buffers.clear()
@@ -72,7 +72,7 @@ class _Rasterize(torch.autograd.Function):
             _, height, width = ctx.shape
             with torch.cuda.device(means.device):
                 state = _fused.raster_vjp_state(means, quats, scales, densities, viewmats, Ks, width, height, beta,
-                                                ctx.eps, ctx.radius_clip, n_isects=ctx.n_isects)
+                                                ctx.eps, ctx.radius_clip)
             context = _vjp_context("rasterize", ctx.shape, primitives,
                                    {"viewmats": viewmats, "Ks": Ks, "state": state}, ctx.eps, ctx.detach_variance)
         g = explicit.rasterize_bwd(context, v_image, v_variance)

@@ -910,7 +910,7 @@ int r2s_raster_emit(const uint16_t* rects, uint32_t C, uint32_t N, uint32_t tile
         uint32_t* vals = arena.take<uint32_t>(size_t(n_isects));
         R2S_REQUIRE(keys && vals, R2S_ERR_WORKSPACE, "intersection workspace too small");
         emit_rects_warp_kernel<<<blocks_for(total, 256), 256, 0, as_stream(stream)>>>(
-            reinterpret_cast<const ushort4*>(rects), uint32_t(total), N, tiles_x, tiles_y, cum_tiles, INT64_MAX, keys,
+            reinterpret_cast<const ushort4*>(rects), uint32_t(total), N, tiles_x, tiles_y, cum_tiles, n_isects, keys,
             vals);
         R2S_TRY(check_launch("raster_emit"));
         const CamLayout cams{cum_tiles, C, N, tiles_x * tiles_y};
@@ -955,7 +955,7 @@ int r2s_isect_tiles_3d_emit(int dtype, const void* means3d, const int32_t* radii
         uint32_t* vals = arena.take<uint32_t>(size_t(n_isects));
         R2S_REQUIRE(keys && vals, R2S_ERR_WORKSPACE, "intersection workspace too small");
         R2S_DISPATCH(dtype, emit_3d_warp_kernel<S><<<blocks_for(N, 256), 256, 0, as_stream(stream)>>>(
-            static_cast<const S*>(means3d), radii, N, tile_size, tiles_x, tiles_y, tiles_z, cum_tiles, INT64_MAX, keys,
+            static_cast<const S*>(means3d), radii, N, tile_size, tiles_x, tiles_y, tiles_z, cum_tiles, n_isects, keys,
             vals));
         R2S_TRY(check_launch("isect_emit_3d"));
         return sort_and_finish(keys, vals, n_isects, n_keys, arena, isect_ids, flatten_ids, offsets,
