@@ -314,7 +314,10 @@ def raster_forward(means, quats, scales, densities, viewmats, Ks, width, height,
                                          means.shape[0], width, height, tile_size, target, kind, weight, image,
                                          variance, device)
     state = RasterState(covars, records, offsets, isect_ids, flatten_ids, ratio, m, width, height, tile_size,
-                        extra={"rects": rects, "cum": cum})
+                        extra={"rects": rects})
+    # The scan (8 bytes a record: 512 MB at 500,000 primitives and 128 views) is kept only for the VJP that reads it.
+    if raster_vjp_takes_tiles(means.dtype, beta is not None, uncertainty is not None, tile_size, width, height, m):
+        state.extra["cum"] = cum
     output = image if uncertainty is None else (image, variance)
     if image_loss is None:
         return output, state
@@ -358,7 +361,7 @@ def _raster_vjp_lists(state: RasterState, dtype, beta: bool, variance: bool):
     form = (dtype, beta, variance, state.tile_size, state.width, state.height)
     if not raster_vjp_takes_tiles(*form, 0):
         return None
-    if state.offsets is not None:
+    if state.offsets is not None and "cum" in state.extra:
         return ((state.flatten_ids, state.offsets, state.extra["cum"], state.n_isects)
                 if raster_vjp_takes_tiles(*form, state.n_isects) else None)
     rects = state.extra["rects"]
@@ -493,6 +496,8 @@ def release_lists(state):
     dropped = [t for t in (state.isect_ids, state.flatten_ids, state.offsets, getattr(state, "packed", None))
                if t is not None]
     state.isect_ids = state.flatten_ids = state.offsets = None
+    if isinstance(state, RasterState) and "cum" in state.extra:
+        dropped.append(state.extra.pop("cum"))
     if hasattr(state, "packed"):
         state.packed = None
     return dropped

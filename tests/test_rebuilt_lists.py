@@ -141,3 +141,18 @@ def test_emission_writes_nothing_past_its_count(device, dims):
     assert bool((ids[m:] == -3).all()) and bool((flat[m:] == -3).all())
     assert bool((ws[nbytes:] == 7).all())
     assert bool((flat[:m] >= 0).all()) and int(offsets.max()) <= m
+
+
+@pytest.mark.gpu
+def test_the_scan_is_kept_only_for_the_vjp_that_reads_it(device):
+    means, quats, scales, dens, q, views, Ks, _, _ = _scene(device)
+    beta = torch.full_like(dens, 1.5)
+    for dtype, options, kept in ((torch.float32, {"uncertainty": q}, True), (torch.float32, {}, False),
+                                 (torch.float32, {"uncertainty": q, "beta": beta}, False),
+                                 (torch.float64, {"uncertainty": q}, False)):
+        args = [t.to(dtype) for t in (means, quats, scales, dens, views, Ks)]
+        _, ctx = r2s.rasterize_fwd(*args, SIZE, **{k: t.to(dtype) for k, t in options.items()})
+        state = ctx.buffers["state"]
+        assert ("cum" in state.extra) == kept
+        explicit.release_intersection_lists(ctx)
+        assert "cum" not in state.extra
