@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(256) raster_slot_reduce_kernel(const Rec2D<flo
         out.c = 0.5f * (-om * s[4]);
         out.o = rec.mu * s[5];
         out.mu = rec.o * s[5];
-        v_unc[r] = om * om * s[6];
+        v_unc[r] = om * (om * s[6]);  // om^2 leaves the range of floats from 1.8e19 on
     } else {
         v_unc[r] = 0.f;
     }

@@ -1464,7 +1464,7 @@ __global__ void __launch_bounds__(kVoxLaneThreads, 4) voxel_bwd_lanes_kernel(
         const float4 o0 = make_float4(-(a * S1 + p * S2 + q * S3), -(bb * S2 + p * S1 + rr * S3),
                                       -(c * S3 + q * S1 + rr * S2), m.s0);
         const float4 o1 = make_float4(0.5f * S11, S12, S13, 0.5f * S22);
-        const float4 o2 = make_float4(S23, 0.5f * S33, 0.f, kVar ? opac * opac * (m.ru.x + m.ru.y) : 0.f);
+        const float4 o2 = make_float4(S23, 0.5f * S33, 0.f, kVar ? opac * (opac * (m.ru.x + m.ru.y)) : 0.f);
         if (!kBulk && sl.slots == nullptr) {
             float* out = reinterpret_cast<float*>(grads + gid);
             red_add_v4(out, o0.x, o0.y, o0.z, o0.w);
