@@ -37,8 +37,8 @@ from .cuda import _backend
 Tensor = torch.Tensor
 RASTER_TILE = 16
 VOXEL_TILE = 8
-# Largest scratch the tile-parallel raster VJP takes for its per-intersection slots (32 bytes each); past it
-# the VJP walks the records' tile rectangles instead.
+# Largest scratch the tile-parallel raster VJP takes for its per-intersection slots (32 bytes each); past it, or where
+# the device has not that much left, the VJP walks the records' tile rectangles instead.
 RASTER_SLOT_BUDGET_BYTES = 8 << 30
 RASTER_SLOT_BYTES = 32
 # Largest scratch the deterministic voxel VJP takes for its per-intersection slots (12 values each);
@@ -353,26 +353,36 @@ def voxel_vjp_state(means, quats, scales, densities, shape, extent, center, beta
 
 
 def _raster_vjp_lists(state: RasterState, dtype, beta: bool, variance: bool):
-    """(flatten_ids, offsets, cum, n_isects) for the tile-parallel VJP, or None where it walks the records.
+    """(flatten_ids, offsets, cum, slots) for the tile-parallel VJP, or None where it walks the records.
 
     Lists that the state does not hold are built from its rectangles and their own count, read here: a count from
-    elsewhere could disagree with the rectangles, and the lists' buffers are sized by it.
+    elsewhere could disagree with the rectangles, and the lists' buffers are sized by it. Where the device has no room
+    for the slots or the rebuilt lists, the record walk takes over, which needs neither.
     """
     form = (dtype, beta, variance, state.tile_size, state.width, state.height)
     if not raster_vjp_takes_tiles(*form, 0):
         return None
-    if state.offsets is not None and "cum" in state.extra:
-        return ((state.flatten_ids, state.offsets, state.extra["cum"], state.n_isects)
-                if raster_vjp_takes_tiles(*form, state.n_isects) else None)
     rects = state.extra["rects"]
-    # Rectangles are in tiles, below 2^13 on this path, so 16-bit differences are exact.
-    x0, y0, x1, y1 = rects.unbind(-1)
-    cum = _raster_scan(((x1 - x0).int() * (y1 - y0)).contiguous())
-    m = _read_total(cum)
-    if not raster_vjp_takes_tiles(*form, m):
+    try:
+        if state.offsets is not None and "cum" in state.extra:
+            flatten_ids, offsets, cum, m = state.flatten_ids, state.offsets, state.extra["cum"], state.n_isects
+            if not raster_vjp_takes_tiles(*form, m):
+                return None
+            return flatten_ids, offsets, cum, _raster_slots(rects.device, m)
+        # Rectangles are in tiles, below 2^13 on this path, so 16-bit differences are exact.
+        x0, y0, x1, y1 = rects.unbind(-1)
+        cum = _raster_scan(((x1 - x0).int() * (y1 - y0)).contiguous())
+        m = _read_total(cum)
+        if not raster_vjp_takes_tiles(*form, m):
+            return None
+        _, flatten_ids, offsets = _raster_lists(rects, cum, m, state.width, state.height, state.tile_size)
+        return flatten_ids, offsets, cum, _raster_slots(rects.device, m)
+    except torch.OutOfMemoryError:
         return None
-    _, flatten_ids, offsets = _raster_lists(rects, cum, m, state.width, state.height, state.tile_size)
-    return flatten_ids, offsets, cum, m
+
+
+def _raster_slots(device, m) -> Tensor:
+    return torch.empty((max(m, 1), RASTER_SLOT_BYTES // 4), dtype=torch.float32, device=device)
 
 
 def raster_backward(state: RasterState, means, quats, scales, densities, beta, uncertainty, viewmats, Ks, eps,
@@ -389,9 +399,9 @@ def raster_backward(state: RasterState, means, quats, scales, densities, beta, u
     rects = state.extra["rects"]
     lists = _raster_vjp_lists(state, means.dtype, beta is not None, v_variance is not None)
     if lists is not None:
-        flatten_ids, offsets, cum, m = lists
+        flatten_ids, offsets, cum, slots = lists
+        m = flatten_ids.numel()
         with _stage("raster_render_bwd"):
-            slots = means.new_empty((max(m, 1), RASTER_SLOT_BYTES // 4))
             _backend.call("r2s_raster_tile_bwd", _ptr(state.records), _ptr(rects), _ptr(uncertainty),
                           int(bool(detach_variance)), _ptr(offsets), _ptr(flatten_ids), m, None,
                           _ptr(cum), _ptr(v_image), _ptr(v_variance), c, n, state.width, state.height,

@@ -144,10 +144,13 @@ def release_intersection_lists(context) -> None:
 
     Not part of the reference's surface: a memory-bounded caller (the serving
     loop's recompute-in-backward mode) calls it between ``rasterize_fwd`` /
-    ``voxelize_fwd`` and the matching backward. The raster VJP rebuilds the
-    lists where it reads them (or walks each record's tile rectangle) and the
-    voxel VJP then walks each primitive's tile box. The gradients are unchanged
-    up to the voxel VJP's summation order.
+    ``voxelize_fwd`` and the matching backward. The raster VJP walks each
+    record's tile rectangle and reads no lists, except for fp32 Gaussians with
+    a variance adjoint: there it builds them again (12 bytes an intersection,
+    16 more while they are sorted, 32 for its slots) and walks the rectangles
+    where the device has no room for that. The voxel VJP then walks each
+    primitive's tile box. The gradients are unchanged up to the summation order
+    of the voxel VJP and of a variance VJP that found no room.
     """
     if not isinstance(context, _Context) or context.used:
         raise RuntimeError("expected an unconsumed explicit context")

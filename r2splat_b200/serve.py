@@ -117,9 +117,9 @@ class ServeStats:
 def lean_step(scene: batched.FitScene, recompute: bool = False):
     """One fit step through the explicit API with transient buffers, then the fused update.
 
-    ``recompute``: free each forward's intersection lists before its backward (the raster VJP never reads
-    them; the voxel VJP then walks the primitives' tile boxes), so the lists of the two passes are never
-    resident at the same time as the backward's buffers.
+    ``recompute``: free each forward's intersection lists before its backward (the raster VJP of an image
+    adjoint alone, as here, never reads them; the voxel VJP then walks the primitives' tile boxes), so the
+    lists of the two passes are never resident at the same time as the backward's buffers.
     """
     cfg = scene.cfg
     _, ctx, v_image, image_loss, _ = explicit.rasterize_fwd_with_loss(

@@ -37,8 +37,8 @@ def test_the_lists_are_sized_by_the_rectangles_own_count(monkeypatch):
     monkeypatch.setattr(torch.cuda.nvtx, "range_pop", lambda: None)
     for stale in (None, 3, 10_000):
         state = _fused.RasterState(None, None, None, None, None, None, stale, 117, 90, 16, extra={"rects": rects})
-        ids, offsets, cum, m = _fused._raster_vjp_lists(state, torch.float32, False, True)
-        assert m == emitted["n"] == ids.numel() == sum(counts)
+        ids, offsets, cum, slots = _fused._raster_vjp_lists(state, torch.float32, False, True)
+        assert emitted["n"] == ids.numel() == slots.shape[0] == sum(counts)
         assert cum.tolist() == torch.tensor(counts).cumsum(0).tolist()
         assert offsets.shape == (2, 6, 8)
 
@@ -156,3 +156,30 @@ def test_the_scan_is_kept_only_for_the_vjp_that_reads_it(device):
         assert ("cum" in state.extra) == kept
         explicit.release_intersection_lists(ctx)
         assert "cum" not in state.extra
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("release", [False, True])
+def test_without_room_for_slots_or_lists_the_records_are_walked(device, monkeypatch, release):
+    """Over the slot budget, or with an allocation refused: the record walk's gradients, bit for bit the same in
+    either case, and the tile walk's to rounding (5e-5 in the relative 2-norm: see the tile walk's own test)."""
+    tiles = _explicit(device, release=release)
+
+    def no_room(*args):
+        raise torch.OutOfMemoryError("no room")
+
+    with monkeypatch.context() as patch:
+        patch.setattr(_fused, "RASTER_SLOT_BUDGET_BYTES", 32)
+        walked = _explicit(device, release=release)
+    for name in ("_raster_slots", "_raster_lists") if release else ("_raster_slots",):
+        with monkeypatch.context() as patch:
+            means, quats, scales, dens, q, views, Ks, v, vv = _scene(device)
+            _, ctx = r2s.rasterize_fwd(means, quats, scales, dens, views, Ks, SIZE, uncertainty=q)
+            if release:
+                explicit.release_intersection_lists(ctx)
+            patch.setattr(_fused, name, no_room)
+            g = r2s.rasterize_bwd(ctx, v, vv)
+        for a, b in zip(walked, (getattr(g, f) for f in FIELDS)):
+            assert torch.equal(a, b)
+    for a, b in zip(walked, tiles):
+        assert float((a - b).norm()) <= 5e-5 * float(a.norm())
