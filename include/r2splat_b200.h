@@ -408,8 +408,9 @@ int r2s_raster_record_bwd(int dtype, const void* records, const uint16_t* rects,
  * over [C,N], and a second pass adds each record's slots in order into grads
  * [C,N,8] (every record written; no atomics). Same adjoints, decisions and null
  * conventions as r2s_raster_record_bwd. n_used: the intersection count kept on
- * the device (capacity-bounded steps), or null; slots past slot_capacity are
- * neither written nor read. records, slots and grads must be 32-byte aligned. */
+ * the device (capacity-bounded steps; 0 where the lists overflowed, which gives
+ * zero gradients), or null; slots past slot_capacity are neither written nor
+ * read. records, slots and grads must be 32-byte aligned. */
 int r2s_raster_tile_bwd(const float* records, const uint16_t* rects, const float* uncertainties,
                         int detach_variance, const int32_t* tile_offsets, const int32_t* flatten_ids,
                         uint64_t n_isects, const int64_t* n_used, const int64_t* tile_cum, const float* v_render,

@@ -344,11 +344,14 @@ __global__ void __launch_bounds__(kTileBwdThreads, kTileBwdBlocksPerSm) raster_t
 // thread per record.
 __global__ void __launch_bounds__(256) raster_slot_reduce_kernel(const Rec2D<float>* __restrict__ records,
                                                                  const int64_t* __restrict__ cum, size_t total,
-                                                                 int64_t capacity, const float* __restrict__ slots,
+                                                                 int64_t capacity, const int64_t* __restrict__ n_dev,
+                                                                 const float* __restrict__ slots,
                                                                  Rec2D<float>* __restrict__ grads,
                                                                  float* __restrict__ v_unc) {
     const size_t r = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (r >= total) return;
+    // Lists that overflowed are empty (*n_dev is 0): no slot was written, and the gradients are zero.
+    if (n_dev != nullptr) capacity = min(capacity, *n_dev);
     const int64_t first = r == 0 ? 0 : min(cum[r - 1], capacity), last = min(cum[r], capacity);
     float s[kSums];
 #pragma unroll
@@ -402,7 +405,7 @@ int launch_tile_bwd(TileBwdGeom g, const Rec2D<float>* rec, const ushort4* rects
                                                                          v_render_var, slots);
     R2S_TRY(check_launch("raster_tile_bwd"));
     raster_slot_reduce_kernel<<<blocks_for(int64_t(total), 256), 256, 0, stream>>>(
-        rec, cum, total, int64_t(g.capacity), slots, grads, v_unc);
+        rec, cum, total, int64_t(g.capacity), g.n_dev, slots, grads, v_unc);
     return check_launch("raster_slot_reduce");
 }
 
