@@ -76,8 +76,8 @@ def _covariances(quats: Tensor, scales: Tensor) -> Tensor:
 
 
 def _read_total(cum: Tensor, before=None) -> int:
-    """The last entry of an inclusive scan. The copy is enqueued first, then ``before`` runs (it waits for work queued
-    earlier), so the device is never idle between the two waits."""
+    """The last entry of an inclusive scan (of any int64 tensor). The copy is enqueued first, then ``before`` runs
+    (it waits for work queued earlier), so the device is never idle between the two waits."""
     host = torch.empty(1, dtype=torch.int64, pin_memory=True)
     done = ctypes.c_void_p()
     _backend.call("r2s_read_count", _ptr(cum) + 8 * (cum.numel() - 1), _ptr(host), ctypes.byref(done),
@@ -88,6 +88,14 @@ def _read_total(cum: Tensor, before=None) -> int:
     finally:
         _backend.call("r2s_wait_done", done)  # the copy writes the pinned word until here
     return ctypes.c_int64.from_address(_ptr(host)).value
+
+
+def _read_sizes(cum: Tensor, counts: Tensor, before=None) -> tuple[int, int]:
+    """(intersections, records that have any) of a scan and its counts; both copies are enqueued before either wait."""
+    nonzero = torch.empty(1, dtype=torch.int64, device=counts.device)
+    _backend.call("r2s_count_nonzero", _ptr(counts), counts.numel(), _ptr(nonzero), _stream(counts.device))
+    visible = []
+    return _read_total(cum, lambda: visible.append(_read_total(nonzero, before))), visible[0]
 
 
 def beta_path_ratio(beta: Tensor) -> Tensor:
@@ -190,19 +198,20 @@ class VoxelState:
 
 
 def raster_intersections(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps, radius_clip,
-                         tile_size=RASTER_TILE, before_count=None):
+                         tile_size=RASTER_TILE, before_count=None, count_visible=False):
     """Projection + packing + sorted tile intersections.
 
-    Returns (records, offsets, isect_ids, flatten_ids, M, rects, cum); rects [C,N,4] are the tile rectangles and
-    cum the inclusive scan of the per-record tile counts, which the VJP's slots are numbered by.
+    Returns (records, offsets, isect_ids, flatten_ids, M, rects, cum, visible); rects [C,N,4] are the tile rectangles,
+    cum the inclusive scan of the per-record tile counts, which the VJP's slots are numbered by, and visible the number
+    of records with tiles (None unless ``count_visible``).
     ``before_count`` runs just before the host reads the intersection count (the pending input checks).
     """
     records, rects, counts = _raster_project(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps,
                                              radius_clip, tile_size)
     cum = _raster_scan(counts)
-    m = _read_total(cum, before_count)
+    m, visible = _read_sizes(cum, counts, before_count) if count_visible else (_read_total(cum, before_count), None)
     isect_ids, flatten_ids, offsets = _raster_lists(rects, cum, m, width, height, tile_size)
-    return records, offsets, isect_ids, flatten_ids, m, rects, cum
+    return records, offsets, isect_ids, flatten_ids, m, rects, cum, visible
 
 
 def _raster_project(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps, radius_clip, tile_size):
@@ -245,18 +254,30 @@ def _raster_lists(rects, cum, m, width, height, tile_size):
     return isect_ids, flatten_ids, offsets
 
 
-def raster_vjp_takes_tiles(dtype, beta: bool, variance: bool, tile_size, width, height, n_slots) -> bool:
-    """Whether the raster VJP runs tile-parallel over the lists (r2s_raster_tile_bwd) rather than record by record.
+def raster_vjp_has_tile_form(dtype, beta: bool, variance: bool, tile_size, width, height) -> bool:
+    """Whether r2s_raster_tile_bwd serves this VJP at all: fp32 Gaussians with a variance adjoint, on tile sizes of
+    whole 8x8 blocks. Without a variance adjoint the record walk keeps the sums' order; compact Beta records are better
+    off with it (boxes of 42 pixels; 0.31 ms by records, 0.46 ms by tiles at 100,000 primitives and 32 views of 384^2).
+    """
+    return (variance and dtype == torch.float32 and not beta and tile_size in (8, 16, 32)
+            and max(width, height) < 65536)
 
-    fp32 Gaussians with a variance adjoint, on tile sizes of whole 8x8 blocks: the tile walk evaluates whole blocks,
-    which pays for Gaussian boxes (317 pixels on average in the cone-beam scene; 1.06 -> 0.57 ms at 50,021 primitives
-    and 17 views of 333 x 517) and not for the compact Beta records (42 pixels; 0.31 ms by records, 0.46 ms by tiles
-    at 100,000 primitives and 32 views of 384^2). Without a variance adjoint the record walk keeps the sums' order.
+
+def raster_vjp_takes_tiles(n_isects, n_visible, n_lists) -> bool:
+    """Whether a VJP that has the tile form takes it: by its intersections, the records that have any, and the lists.
+
+    The tile walk evaluates whole 8x8 blocks at 0.11 ns a pair, the record walk the pixels of each record's box at some
+    0.075 ns a pair for each tile that the record meets, so tiles pay once a record meets 2.25 of them on average
+    (us by records / by tiles: 2.08 tiles a record 102 / 120, 2.21 202 / 226, 2.35 1564 / 1329, 2.9 1489 / 1186, 4.4
+    984 / 537, 7.8 511 / 286, 29 1132 / 361). A list costs 2.1 ns by itself, its tile's adjoints being staged however
+    short it is: 65,536 lists of 4, 9 and 18 records of 3.7 tiles take 164, 207 and 271 us against 81, 163 and 277 by
+    records. Up to 4,096 lists that is below the record walk's own latency (1,000 records on 1,024 lists: 63 / 19).
     The rule depends on the scene alone, not on whether the lists are still held, so a rebuilt backward gives the same
     gradients.
     """
-    return (variance and dtype == torch.float32 and not beta and tile_size in (8, 16, 32)
-            and max(width, height) < 65536 and n_slots * RASTER_SLOT_BYTES <= RASTER_SLOT_BUDGET_BYTES)
+    return (4 * n_isects >= 9 * n_visible
+            and n_isects * (2 * n_isects - 3 * n_visible) >= 56 * n_visible * max(n_lists - 4096, 0)
+            and n_isects * RASTER_SLOT_BYTES <= RASTER_SLOT_BUDGET_BYTES)
 
 
 IMAGE_LOSS_KINDS = {"mse": 0, "l1": 1}  # R2S_IMAGE_LOSS_MSE, R2S_IMAGE_LOSS_L1
@@ -295,9 +316,11 @@ def raster_forward(means, quats, scales, densities, viewmats, Ks, width, height,
     c = viewmats.shape[0]
     covars = _covariances(quats, scales)
     ratio = beta_path_ratio(beta) if beta is not None else None
-    records, offsets, isect_ids, flatten_ids, m, rects, cum = raster_intersections(
+    has_tile_vjp = raster_vjp_has_tile_form(means.dtype, beta is not None, uncertainty is not None, tile_size, width,
+                                            height)
+    records, offsets, isect_ids, flatten_ids, m, rects, cum, visible = raster_intersections(
         means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps, radius_clip, tile_size,
-        before_count)
+        before_count, has_tile_vjp)
     image = means.new_empty((c, height, width))
     variance = torch.empty_like(image) if uncertainty is not None else None
     tx = (width + tile_size - 1) // tile_size
@@ -316,8 +339,8 @@ def raster_forward(means, quats, scales, densities, viewmats, Ks, width, height,
     state = RasterState(covars, records, offsets, isect_ids, flatten_ids, ratio, m, width, height, tile_size,
                         extra={"rects": rects})
     # The scan (8 bytes a record: 512 MB at 500,000 primitives and 128 views) is kept only for the VJP that reads it.
-    if raster_vjp_takes_tiles(means.dtype, beta is not None, uncertainty is not None, tile_size, width, height, m):
-        state.extra["cum"] = cum
+    if has_tile_vjp:
+        state.extra.update(cum=cum, visible=visible)
     output = image if uncertainty is None else (image, variance)
     if image_loss is None:
         return output, state
@@ -359,23 +382,27 @@ def _raster_vjp_lists(state: RasterState, dtype, beta: bool, variance: bool):
     elsewhere could disagree with the rectangles, and the lists' buffers are sized by it. Where the device has no room
     for the slots or the rebuilt lists, the record walk takes over, which needs neither.
     """
-    form = (dtype, beta, variance, state.tile_size, state.width, state.height)
-    if not raster_vjp_takes_tiles(*form, 0):
+    if not raster_vjp_has_tile_form(dtype, beta, variance, state.tile_size, state.width, state.height):
         return None
     rects = state.extra["rects"]
+    tx, ty = ((size + state.tile_size - 1) // state.tile_size for size in (state.width, state.height))
+    n_lists = rects.shape[0] * ty * tx
     try:
-        if state.offsets is not None and "cum" in state.extra:
-            flatten_ids, offsets, cum, m = state.flatten_ids, state.offsets, state.extra["cum"], state.n_isects
-            if not raster_vjp_takes_tiles(*form, m):
-                return None
-            return flatten_ids, offsets, cum, _raster_slots(rects.device, m)
-        # Rectangles are in tiles, below 2^13 on this path, so 16-bit differences are exact.
-        x0, y0, x1, y1 = rects.unbind(-1)
-        cum = _raster_scan(((x1 - x0).int() * (y1 - y0)).contiguous())
-        m = _read_total(cum)
-        if not raster_vjp_takes_tiles(*form, m):
+        held = state.offsets is not None and "cum" in state.extra
+        if held:
+            cum, m, visible = state.extra["cum"], state.n_isects, state.extra["visible"]
+        else:
+            # Rectangles are in tiles, below 2^13 on this path, so 16-bit differences are exact.
+            x0, y0, x1, y1 = rects.unbind(-1)
+            counts = ((x1 - x0).int() * (y1 - y0)).contiguous()
+            cum = _raster_scan(counts)
+            m, visible = _read_sizes(cum, counts)
+        if not raster_vjp_takes_tiles(m, visible, n_lists):
             return None
-        _, flatten_ids, offsets = _raster_lists(rects, cum, m, state.width, state.height, state.tile_size)
+        if held:
+            flatten_ids, offsets = state.flatten_ids, state.offsets
+        else:
+            _, flatten_ids, offsets = _raster_lists(rects, cum, m, state.width, state.height, state.tile_size)
         return flatten_ids, offsets, cum, _raster_slots(rects.device, m)
     except torch.OutOfMemoryError:
         return None

@@ -514,6 +514,23 @@ __device__ __forceinline__ void block_scatter_ballot(const uint32_t* __restrict_
     }
 }
 
+// The number of nonzero counts, added up block by block (whole numbers: any order gives the same sum).
+__global__ void __launch_bounds__(256) count_nonzero_kernel(const int32_t* __restrict__ counts, uint64_t n,
+                                                            unsigned long long* __restrict__ out) {
+    uint32_t mine = 0u;
+    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) mine += counts[i] != 0;
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    __shared__ uint32_t s_sum[8];
+    if ((threadIdx.x & 31u) == 0u) s_sum[threadIdx.x >> 5] = mine;
+    __syncthreads();
+    if (threadIdx.x == 0u) {
+        uint32_t sum = 0u;
+        for (int w = 0; w < 8; ++w) sum += s_sum[w];
+        if (sum != 0u) atomicAdd(out, static_cast<unsigned long long>(sum));
+    }
+}
+
 // ------------------------------------------------ camera-segmented 2D sort
 //
 // 2D keys are cam * n_tiles + tile and emission is camera-major, so the key
@@ -849,6 +866,17 @@ int r2s_scan_tile_counts(const int32_t* counts, uint64_t n, int64_t* cum, void* 
                          void* stream) {
     return device_scan<int32_t, int64_t, true>(counts, cum, int64_t(n), workspace, workspace_bytes,
                                                as_stream(stream));
+}
+
+int r2s_count_nonzero(const int32_t* counts, uint64_t n, int64_t* out, void* stream) {
+    R2S_REQUIRE(out != nullptr && (counts != nullptr || n == 0), R2S_ERR_ARGUMENT, "counts and out must be non-null");
+    cudaStream_t st = as_stream(stream);
+    if (cudaMemsetAsync(out, 0, sizeof(int64_t), st) != cudaSuccess) return fail(R2S_ERR_CUDA, "memset failed");
+    if (n == 0) return R2S_OK;
+    const uint64_t blocks = (n + 2047) / 2048;  // eight counts a thread, up to eight blocks a SM
+    count_nonzero_kernel<<<unsigned(blocks < 1184 ? blocks : 1184), 256, 0, st>>>(
+        counts, n, reinterpret_cast<unsigned long long*>(out));
+    return check_launch("count_nonzero");
 }
 
 size_t r2s_isect_emit_workspace(uint64_t n_isects, uint64_t n_keys) {

@@ -395,11 +395,14 @@ int launch_tile_bwd(TileBwdGeom g, const Rec2D<float>* rec, const ushort4* rects
     // A list is shared by several CTAs when there are too few lists to fill the chip: about 8192 CTAs (eleven
     // waves), as far as a warp keeps eight records. Measured on the walk without the variance terms: one view of
     // 100,000 primitives at 512^2 (1024 lists of 360) 0.112, 0.089, 0.063, 0.060 and 0.069 ms with 1, 2, 4, 8 and
-    // 16 CTAs a list; 65,536 lists of 720 4.57 ms with one or two and 4.79 ms with four.
+    // 16 CTAs a list; 65,536 lists of 720 4.57 ms with one or two and 4.79 ms with four. A few long lists need more:
+    // one view at 64^2 (16 lists of 14,000, with the variance) 0.124, 0.068 and 0.062 ms with 16, 64 and 256 CTAs a
+    // list, at 100^2 (49 lists of 6,300) 0.155, 0.071 and 0.066 (60 CTAs of 64 records beat 250 of 8 on 16 lists of
+    // 2,850: 0.029 / 0.031).
     const uint64_t lists = uint64_t(g.n_tiles) * g.C;
     const uint64_t mean = (g.n_dev != nullptr ? g.capacity : uint64_t(g.n_isects)) / lists;
     const uint64_t fill = (8192 + lists - 1) / lists, records = (mean + 8 * kTileBwdWarps - 1) / (8 * kTileBwdWarps);
-    const unsigned split = unsigned(std::min<uint64_t>(16u, std::max<uint64_t>(1u, std::min(fill, records))));
+    const unsigned split = unsigned(std::min<uint64_t>(64u, std::max<uint64_t>(1u, std::min(fill, records))));
     const dim3 grid(g.n_tiles, g.C, split);
     raster_tile_bwd_kernel<<<grid, kTileBwdThreads, smem, stream>>>(rec, meta, var_q, offsets, ids, g, v_render,
                                                                          v_render_var, slots);

@@ -32,7 +32,7 @@ def test_the_lists_are_sized_by_the_rectangles_own_count(monkeypatch):
     monkeypatch.setattr(_fused._backend, "library", lambda: type("L", (), {
         "r2s_isect_emit_workspace": staticmethod(lambda m, keys: m)})())
     monkeypatch.setattr(_fused, "_raster_scan", lambda c: c.flatten().to(torch.int64).cumsum(0))
-    monkeypatch.setattr(_fused, "_read_total", lambda cum: int(cum[-1]))
+    monkeypatch.setattr(_fused, "_read_sizes", lambda cum, counts: (int(cum[-1]), int((counts != 0).sum())))
     monkeypatch.setattr(torch.cuda.nvtx, "range_push", lambda name: None)
     monkeypatch.setattr(torch.cuda.nvtx, "range_pop", lambda: None)
     for stale in (None, 3, 10_000):
@@ -183,3 +183,46 @@ def test_without_room_for_slots_or_lists_the_records_are_walked(device, monkeypa
             assert torch.equal(a, b)
     for a, b in zip(walked, tiles):
         assert float((a - b).norm()) <= 5e-5 * float(a.norm())
+
+
+def test_rule_for_the_tile_walk():
+    takes = _fused.raster_vjp_takes_tiles
+    assert takes(0, 0, 10**6)  # nothing to walk
+    assert takes(9, 4, 4096) and not takes(8, 4, 4096)  # 2.25 tiles a record
+    # 65,536 lists of 3.7 tiles a record: 18 records a list pay for the lists, nine do not.
+    assert takes(65536 * 18, 65536 * 18 * 10 // 37, 65536) and not takes(65536 * 9, 65536 * 9 * 10 // 37, 65536)
+    budget = _fused.RASTER_SLOT_BUDGET_BYTES // _fused.RASTER_SLOT_BYTES
+    assert takes(budget, 1000, 1) and not takes(budget + 1, 1000, 1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [0, 1, 255, 2049, 3_000_001])
+def test_records_with_tiles_are_counted(device, n):
+    counts = torch.randint(-1, 3, (n,), generator=torch.Generator().manual_seed(n)).to(device, torch.int32)
+    out = torch.full((1,), 99, dtype=torch.int64, device=device)
+    _backend.call("r2s_count_nonzero", _ptr(counts), n, _ptr(out), _fused._stream(device))
+    assert int(out) == int((counts != 0).sum())
+
+
+@pytest.mark.gpu
+def test_small_footprints_take_the_record_walk(device, monkeypatch):
+    """Records of about one tile each: the gradients of the record walk, bit for bit, kept, released or recomputed."""
+    original = _scene
+
+    def small(device, n=3000, cameras=5):
+        scene = original(device, n, cameras)
+        scene[2] = scene[2] * 0.02
+        return scene
+
+    monkeypatch.setitem(globals(), "_scene", small)
+    kept = _explicit(device)
+    leaves, _, loss = _graph(device, True)
+    others = [_explicit(device, release=True), torch.autograd.grad(loss, leaves)]
+    monkeypatch.setattr(_fused, "raster_vjp_takes_tiles", lambda *args: False)
+    others.append(_explicit(device))
+    monkeypatch.setattr(_fused, "raster_vjp_takes_tiles", lambda *args: True)
+    tiles = _explicit(device)
+    for other in others:
+        for a, b in zip(kept, other):
+            assert torch.equal(a, b)
+    assert not all(torch.equal(a, b) for a, b in zip(kept, tiles))
