@@ -599,7 +599,8 @@ int r2s_voxel_record_bwd(int dtype, const void* records, const void* means_v, co
  *                       v_render = lambda * sign(render - target) / numel
  *                       (image_loss_l1_bwd with grad_output = 1).
  * loss_value = the mean without lambda. n_used, when non-NULL, overrides
- * n_isects (capacity-bounded mode). Workspace:
+ * n_isects (capacity-bounded mode), which may then give the capacity, as a
+ * guess of the lists' length for the choice of kernel, or 0. Workspace:
  * r2s_raster_image_loss_workspace(C, tiles_x, tiles_y). render must not
  * alias target or v_render. */
 #define R2S_IMAGE_LOSS_MSE 0

@@ -262,8 +262,8 @@ class FitScene:
                           _p(self.flatten_ids), _p(self.offsets), _p(self.emit_ws), self.emit_ws.numel(), s)
             # Tile forward with the MSE image loss and its gradient in the epilogue.
             _backend.call("r2s_raster_render_image_loss", d, _p(self.records), None, beta_flag, _p(self.offsets),
-                          _p(self.flatten_ids), 0, _p(self.n_used), self.c, self.n, self.width, self.height,
-                          self.cfg.tile, self.tx, self.ty, self.cfg.stage_batch, _p(self.target), 0, 1.0,
+                          _p(self.flatten_ids), self.capacity_2d, _p(self.n_used), self.c, self.n, self.width,
+                          self.height, self.cfg.tile, self.tx, self.ty, self.cfg.stage_batch, _p(self.target), 0, 1.0,
                           _p(self.image), None, _p(self.v_image), _p(self.image_loss), _p(self.image_loss_value),
                           _p(self.image_loss_ws), self.image_loss_ws.numel(), s)
             _backend.call("r2s_raster_record_bwd", d, _p(self.records), _p(self.rects), None, beta_flag, 0,

@@ -1413,8 +1413,15 @@ int launch_fwd_p(const RasterGeom& g, const Rec2D<S>* rec, const S* unc, const i
         // of 256^2, 40,000 Gaussians 0.246 / 0.138 (tile 8), 0.179 / 0.115 (16), 0.262 / 0.207 (32); 32 views of
         // 384^2, 100,000 Beta 0.81 / 0.25, 0.364 / 0.240, 0.524 / 0.428. At tile 32 a few lists are better off
         // with the pair kernel's 16 warps a tile (16 lists of 340: 0.042 / 0.050).
+        // Lists of fewer than twelve records on average go to the pair kernel at tile 16: the group kernel's fixed part
+        // (three larger buffers, a list per group) is what such a launch costs. 65,536 lists of 1.8, 5.4, 11 and 14
+        // Gaussians, us pair / group: 81 / 104, 100 / 118, 130 / 139, 149 / 152; with the variance 94 / 112 and 173 /
+        // 169 at 1.8 and 14; Beta 89 / 99 and 138 / 127 at 1.8 and 14. Tiles of 8 and 32 gain at every length (1.0
+        // records a list 257 / 144 at tile 8, 4.2 92 / 56 at tile 32). A count that only the device knows, with no
+        // capacity given beside it, is taken for long lists.
         const uint64_t lists = uint64_t(g.tiles_x) * g.tiles_y * g.C;
-        if (lists < (uint64_t(1) << 31)) {
+        const bool short_lists = g.T == 16 && (g.n_dev == nullptr || g.n_isects != 0) && g.n_isects < 12 * lists;
+        if (lists < (uint64_t(1) << 31) && !short_lists) {
             if (g.T == 8)
                 return launch_fwd_group<kBeta, kVar, 8, 4>(g, rec, unc, offsets, ids, out, out_var, loss, 64u, stream);
             if (g.T == 16)
@@ -1790,7 +1797,7 @@ int r2s_raster_render_capacity(int dtype, const void* records, const void* uncer
                                uint32_t tiles_x, uint32_t tiles_y, uint32_t stage_batch, void* render,
                                void* render_var, void* stream) {
     R2S_REQUIRE(n_used != nullptr, R2S_ERR_ARGUMENT, "n_used must be non-null");
-    RasterGeom g{C, N, 1u, width, height, tile_size, tiles_x, tiles_y};
+    RasterGeom g{C, N, 0u, width, height, tile_size, tiles_x, tiles_y};
     g.n_dev = n_used;
     if (stage_batch != 0) g.stage_batch = stage_batch;
     R2S_DISPATCH(dtype, return launch_fwd<S>(g, static_cast<const Rec2D<S>*>(records),
