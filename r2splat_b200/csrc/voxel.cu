@@ -419,25 +419,27 @@ __device__ __forceinline__ BoxWalk box_walk(const Rec3D<float>& r, uint32_t ox, 
 // record's two or three steps (some 130 instructions) and their latency.
 // 100,000 primitives in 192^3 (0.44 M pairs): 0.172 -> 0.057 ms; 500,000 with
 // the variance in 384^3 (5.3 M): 1.97 -> 0.99 ms (every voxel of the tile
-// evaluated before). A needle's box can be the whole tile, which costs what it
-// did.
+// evaluated before).
+//
+// kSlabs warps share a tile, each with its own z-slab of it, where there are too
+// few tiles to fill the chip; each walks the whole list.
 constexpr int kVoxBetaWarps = 2;
-// Grids of at most three tiles per SM keep the forms with several warps a tile (216 tiles: 0.019 / 0.021 ms forward,
-// 0.020 / 0.025 VJP; 512 tiles 0.025 / 0.023 and 0.027 / 0.027; 1,728 tiles 0.060 / 0.025 and 0.056 / 0.031).
+// Grids of at most three tiles per SM keep the forms with several warps a tile.
 constexpr uint32_t kVoxBetaTiles = 444;
 
-template <bool kVar, bool kBulk>
+template <bool kVar, bool kBulk, uint32_t kSlabs>
 __global__ void __launch_bounds__(32 * kVoxBetaWarps) voxel_beta_fwd_kernel(
     const Rec3D<float>* __restrict__ records, const int32_t* __restrict__ offsets,
     const int32_t* __restrict__ flatten_ids, VoxelGeom g, float* __restrict__ volume, float* __restrict__ volume_var) {
-    constexpr uint32_t T = 8u;
-    __shared__ float s_accs[kVoxBetaWarps][T * T * T];
-    __shared__ float s_accvs[kVoxBetaWarps][kVar ? T * T * T : 1];
+    constexpr uint32_t T = 8u, kPlanes = T / kSlabs, kVoxels = T * T * kPlanes;
+    __shared__ float s_accs[kVoxBetaWarps][kVoxels];
+    __shared__ float s_accvs[kVoxBetaWarps][kVar ? kVoxels : 1];
     __shared__ Rec3D<float> s_recs[kVoxBetaWarps][32];
     __shared__ BoxWalk s_boxes[kVoxBetaWarps][32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t n_tiles = g.tiles_x * g.tiles_y * g.tiles_z;
-    const uint32_t key = blockIdx.x * kVoxBetaWarps + warp;
+    const uint32_t at_warp = blockIdx.x * kVoxBetaWarps + warp;
+    const uint32_t key = at_warp / kSlabs, slab = at_warp % kSlabs;
     if (key >= n_tiles) return;
     float* s_acc = s_accs[warp];
     float* s_accv = s_accvs[warp];
@@ -446,14 +448,14 @@ __global__ void __launch_bounds__(32 * kVoxBetaWarps) voxel_beta_fwd_kernel(
     const uint32_t tz = key / (g.tiles_x * g.tiles_y);
     const uint32_t rem = key - tz * g.tiles_x * g.tiles_y;
     const uint32_t ty = rem / g.tiles_x, tx = rem - ty * g.tiles_x;
-    const uint32_t ox = tx * T, oy = ty * T, oz = tz * T;
+    const uint32_t ox = tx * T, oy = ty * T, oz = tz * T + slab * kPlanes;  // the warp's slab of the tile
     if (ox >= g.dim2 || oy >= g.dim1 || oz >= g.dim0) return;
-    const uint32_t vx = min(T, g.dim2 - ox), vy = min(T, g.dim1 - oy), vz = min(T, g.dim0 - oz);
+    const uint32_t vx = min(T, g.dim2 - ox), vy = min(T, g.dim1 - oy), vz = min(kPlanes, g.dim0 - oz);
     const int32_t start = offsets[key];
     const int32_t n_total = g.n_dev != nullptr ? int32_t(*g.n_dev) : int32_t(g.n_isects);
     const int32_t end = (key + 1 == n_tiles) ? n_total : offsets[key + 1];
 #pragma unroll
-    for (uint32_t i = 0; i < T * T * T; i += 32u) {
+    for (uint32_t i = 0; i < kVoxels; i += 32u) {
         s_acc[i + lane] = 0.f;
         if (kVar) s_accv[i + lane] = 0.f;
     }
@@ -475,6 +477,15 @@ __global__ void __launch_bounds__(32 * kVoxBetaWarps) voxel_beta_fwd_kernel(
             live &= live - 1u;
             const Rec3D<float> r = s_rec[s];
             const BoxWalk box = s_box[s];
+            auto add_sample = [&](uint32_t at, float qf) {
+                if (!(qf < 0.f || qf >= 1.f)) {
+                    const float alpha = r.o * pow(1.f - qf, r.beta);
+                    if (!(fabsf(alpha) < 1e-5f)) {
+                        s_acc[at] += alpha;
+                        if (kVar) s_accv[at] = fmaf(__fmul_rn(r.q, alpha), alpha, s_accv[at]);
+                    }
+                }
+            };
             for (uint32_t k = lane; k < box.area; k += 32u) {
                 const uint32_t row = (k * box.magic_w) >> 16, x = k - row * box.w;
                 const uint32_t z = (row * box.magic_h) >> 16, y = row - z * box.h;
@@ -486,20 +497,14 @@ __global__ void __launch_bounds__(32 * kVoxBetaWarps) voxel_beta_fwd_kernel(
                 const float qf = fmaf(__fmul_rn(__fmul_rn(2.f, r.c12), d2), d3,
                                       fmaf(__fmul_rn(__fmul_rn(2.f, r.c02), d1), d3,
                                            fmaf(__fmul_rn(__fmul_rn(2.f, r.c01), d1), d2, sq)));
-                if (!(qf < 0.f || qf >= 1.f)) {
-                    const float alpha = r.o * pow(1.f - qf, r.beta);
-                    if (!(fabsf(alpha) < 1e-5f)) {
-                        s_acc[at] += alpha;
-                        if (kVar) s_accv[at] = fmaf(__fmul_rn(r.q, alpha), alpha, s_accv[at]);
-                    }
-                }
+                add_sample(at, qf);
             }
             __syncwarp();  // the next record's lanes add to the same voxels
         }
     }
     __syncwarp();
 #pragma unroll
-    for (uint32_t i = 0; i < T * T * T; i += 32u) {
+    for (uint32_t i = 0; i < kVoxels; i += 32u) {
         const uint32_t at = i + lane, x = at & 7u, y = (at >> 3) & 7u, z = at >> 6;
         if (x < vx && y < vy && z < vz) {
             const size_t vid = (size_t(oz + z) * g.dim1 + (oy + y)) * g.dim2 + (ox + x);
@@ -1498,7 +1503,8 @@ template <bool kVar, bool kBulk>
 __global__ void __launch_bounds__(32 * kVoxBetaWarps, 10) voxel_beta_bwd_kernel(
     const Rec3D<float>* __restrict__ records, bool chain_var, const int32_t* __restrict__ offsets,
     const int32_t* __restrict__ flatten_ids, VoxelGeom g, const float* __restrict__ v_volume,
-    const float* __restrict__ v_volume_var, Rec3D<float>* __restrict__ grads, VoxelSlots<float> sl) {
+    const float* __restrict__ v_volume_var, Rec3D<float>* __restrict__ grads, VoxelSlots<float> sl,
+    uint32_t shares) {
     constexpr uint32_t T = 8u;
     __shared__ float s_gs[kVoxBetaWarps][T * T * T];
     __shared__ float s_us[kVoxBetaWarps][kVar ? T * T * T : 1];
@@ -1506,7 +1512,8 @@ __global__ void __launch_bounds__(32 * kVoxBetaWarps, 10) voxel_beta_bwd_kernel(
     __shared__ BoxWalk s_boxes[kVoxBetaWarps][32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t n_tiles = g.tiles_x * g.tiles_y * g.tiles_z;
-    const uint32_t key = blockIdx.x * kVoxBetaWarps + warp;
+    const uint32_t at_warp = blockIdx.x * kVoxBetaWarps + warp;
+    const uint32_t key = at_warp / shares;
     if (key >= n_tiles) return;
     float* s_g = s_gs[warp];
     float* s_u = s_us[warp];
@@ -1518,9 +1525,13 @@ __global__ void __launch_bounds__(32 * kVoxBetaWarps, 10) voxel_beta_bwd_kernel(
     const uint32_t ox = tx * T, oy = ty * T, oz = tz * T;
     if (ox >= g.dim2 || oy >= g.dim1 || oz >= g.dim0) return;
     const uint32_t vx = min(T, g.dim2 - ox), vy = min(T, g.dim1 - oy), vz = min(T, g.dim0 - oz);
-    const int32_t start = offsets[key];
+    const int32_t first = offsets[key];
     const int32_t n_total = g.n_dev != nullptr ? int32_t(*g.n_dev) : int32_t(g.n_isects);
-    const int32_t end = (key + 1 == n_tiles) ? n_total : offsets[key + 1];
+    const int32_t last = (key + 1 == n_tiles) ? n_total : offsets[key + 1];
+    // The warp's share of the list, whole steps of four pairs.
+    const int64_t share = (int64_t(last - first) + 4 * shares - 1) / (4 * shares) * 4;
+    const int64_t from = first + share * (at_warp % shares);
+    const int32_t start = int32_t(min(from, int64_t(last))), end = int32_t(min(from + share, int64_t(last)));
     if (end <= start) return;
 #pragma unroll 4
     for (uint32_t i = 0; i < T * T * T; i += 32u) {
@@ -2198,10 +2209,20 @@ int launch_vfwd_p(const VoxelGeom& g, const Rec3D<S>* rec, const int32_t* offset
         }
     }
     if constexpr (kBeta && std::is_same<S, float>::value) {
-        if (g.T == 8 && g.tiles_x * g.tiles_y * g.tiles_z > kVoxBetaTiles) {
-            voxel_beta_fwd_kernel<kVar, kBulk>
-                <<<blocks_for(g.tiles_x * g.tiles_y * g.tiles_z, kVoxBetaWarps), 32 * kVoxBetaWarps, 0, stream>>>(
-                    rec, offsets, ids, g, vol, vol_var);
+        // Four slabs a tile up to eight tiles a SM, two up to 24 (general kernel us, then its multiples with 1, 2 and 4
+        // slabs: 512 tiles, lists of 374 small boxes 98, 0.78, 0.53, 0.43, of 76 boxes of whole tiles 31, 2.25, 1.38,
+        // 1.00; 1,728 tiles, 144 small 103, 0.40, 0.34, 0.44, 52 whole 48, 1.37, 0.96, 1.02; 4,096 tiles, 76 small 119,
+        // 0.29, 0.36, 0.48, 42 whole 79, 0.96, 0.89, 0.97).
+        const uint32_t n_tiles = g.tiles_x * g.tiles_y * g.tiles_z;
+        if (g.T == 8 && n_tiles > kVoxBetaTiles) {
+            const uint32_t slabs = n_tiles <= 1184u ? 4u : n_tiles <= 3552u ? 2u : 1u;
+            const unsigned grid = blocks_for(int64_t(n_tiles) * slabs, kVoxBetaWarps), threads = 32 * kVoxBetaWarps;
+            if (slabs == 4u)
+                voxel_beta_fwd_kernel<kVar, kBulk, 4u><<<grid, threads, 0, stream>>>(rec, offsets, ids, g, vol, vol_var);
+            else if (slabs == 2u)
+                voxel_beta_fwd_kernel<kVar, kBulk, 2u><<<grid, threads, 0, stream>>>(rec, offsets, ids, g, vol, vol_var);
+            else
+                voxel_beta_fwd_kernel<kVar, kBulk, 1u><<<grid, threads, 0, stream>>>(rec, offsets, ids, g, vol, vol_var);
             return check_launch("voxelize_to_voxels_fwd");
         }
     }
@@ -2229,6 +2250,21 @@ int launch_vfwd(const VoxelGeom& g, const Rec3D<S>* rec, bool beta, const int32_
                : launch_vfwd_p<S, false, false, false>(g, rec, offsets, ids, vol, vol_var, stream);
 }
 
+// Warps that share a tile's list in voxel_beta_bwd_kernel, or 0 where voxel_bwd_kernel's eight warps a tile are faster:
+// few tiles with short lists, or records that reach most of a tile (more than 16 tiles each). voxel_bwd_kernel us, then its
+// multiples with 1, 2 and 4 warps (pairs a tile, small boxes unless said otherwise): 512 tiles 38 pairs 15, 1.78, 1.18,
+// 1.06, 374 pairs 67, 1.34, 0.87, 0.61, 76 of whole tiles 34, 3.0, 1.9, 1.2; 1,728 tiles 18 pairs 27, 1.03, 1.05, 1.16,
+// 48 pairs 40, 0.91, 0.83, 0.88, 373 middling 240, 1.12, 1.02, 0.92, 52 of whole tiles 71, 1.35, 1.17, 1.16; 4,096 tiles
+// 12 pairs 51, 0.77, 0.93, 1.06, 239 middling 395, 1.12, 0.99, 0.98, 42 of whole tiles 141, 1.06, 0.94, 1.05; 15,625
+// tiles 29 pairs 247, 0.49, 0.58, 0.82.
+inline uint32_t beta_bwd_shares(uint64_t tiles, uint64_t pairs, uint64_t n) {
+    const bool large = pairs > 16 * n;
+    if (tiles <= kVoxBetaTiles) return 0u;
+    if (tiles <= 1480u) return pairs >= 128 * tiles ? 4u : 0u;
+    if (tiles <= 3552u) return pairs >= 128 * tiles ? 4u : large ? 0u : pairs >= 32 * tiles ? 2u : 1u;
+    return pairs >= 64 * tiles || (large && tiles <= 5920u) ? 2u : 1u;
+}
+
 template <typename S, bool kBeta, bool kVar, bool kBulk>
 int launch_vbwd_p(const VoxelGeom& g, const Rec3D<S>* rec, bool chain_var, const int32_t* offsets,
                   const int32_t* ids, const S* v_vol, const S* v_vol_var, Rec3D<S>* grads, cudaStream_t stream,
@@ -2242,10 +2278,14 @@ int launch_vbwd_p(const VoxelGeom& g, const Rec3D<S>* rec, bool chain_var, const
         }
     }
     if constexpr (std::is_same<S, float>::value && kBeta) {
-        if (g.T == 8 && g.tiles_x * g.tiles_y * g.tiles_z > kVoxBetaTiles) {
+        // With the count on the device, the slots' capacity stands for it.
+        const uint64_t n_tiles = uint64_t(g.tiles_x) * g.tiles_y * g.tiles_z;
+        const uint64_t pairs = g.n_dev == nullptr ? g.n_isects : sl.slots != nullptr ? sl.capacity : 0u;
+        const uint32_t shares = g.T == 8 ? beta_bwd_shares(n_tiles, pairs, g.N) : 0u;
+        if (shares != 0u) {
             voxel_beta_bwd_kernel<kVar, kBulk>
-                <<<blocks_for(g.tiles_x * g.tiles_y * g.tiles_z, kVoxBetaWarps), 32 * kVoxBetaWarps, 0, stream>>>(
-                    rec, chain_var, offsets, ids, g, v_vol, v_vol_var, grads, sl);
+                <<<blocks_for(int64_t(n_tiles) * shares, kVoxBetaWarps), 32 * kVoxBetaWarps, 0, stream>>>(
+                    rec, chain_var, offsets, ids, g, v_vol, v_vol_var, grads, sl, shares);
             return check_launch("voxelize_to_voxels_bwd");
         }
     }
