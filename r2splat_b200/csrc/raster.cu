@@ -1156,12 +1156,14 @@ __device__ __forceinline__ void walk_record_groups(uint32_t sorted, uint32_t p, 
 }
 
 // Blocks per SM the record VJP is compiled for: three (80 registers) for fp32. Two (122) or four (64, with spills for
-// the packed walk) are slower; the Beta variance form would take two on its own.
-template <typename S>
-constexpr int kRecBwdMinBlocks = sizeof(S) == 4 ? 3 : 0;
+// the packed walk) are slower; the Beta variance form would take two on its own. Gaussians with the variance take four:
+// what comes here of them are small boxes, whose walks are short (500,000 records of a few pixels in 8 views of 256^2:
+// 0.345 ms with three, 0.305 with four; 50,021 of 317 pixels in 17 views 0.98 / 1.04).
+template <typename S, bool kBeta, bool kVar, bool kAbs>
+constexpr int kRecBwdMinBlocks = sizeof(S) != 4 ? 0 : !kBeta && kVar && !kAbs ? 4 : 3;
 
 template <typename S, bool kBeta, bool kVar, bool kAbs>
-__global__ void __launch_bounds__(kRecBwdThreads, kRecBwdMinBlocks<S>) raster_record_bwd_kernel(
+__global__ void __launch_bounds__(kRecBwdThreads, (kRecBwdMinBlocks<S, kBeta, kVar, kAbs>)) raster_record_bwd_kernel(
     const Rec2D<S>* __restrict__ records, const ushort4* __restrict__ rects, const S* __restrict__ var_q,
     uint32_t C, uint32_t N, uint32_t width, uint32_t height, uint32_t T, const S* __restrict__ v_render,
     const S* __restrict__ v_render_var, Rec2D<S>* __restrict__ grads, S* __restrict__ v_abs,
