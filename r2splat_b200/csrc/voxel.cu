@@ -2302,8 +2302,16 @@ template <typename S, bool kBeta, bool kVar, bool kBulk>
 int launch_vbwd_p(const VoxelGeom& g, const Rec3D<S>* rec, bool chain_var, const int32_t* offsets,
                   const int32_t* ids, const S* v_vol, const S* v_vol_var, Rec3D<S>* grads, cudaStream_t stream,
                   const VoxelSlots<S>& sl) {
+    // With the count on the device, the slots' capacity stands for it.
+    const uint64_t n_tiles = uint64_t(g.tiles_x) * g.tiles_y * g.tiles_z;
+    const uint64_t pairs = g.n_dev == nullptr ? g.n_isects : sl.slots != nullptr ? sl.capacity : 0u;
     if constexpr (std::is_same<S, float>::value && !kBeta) {
-        if (g.T == 8) {
+        // A lane per pair walks the whole tile, which short lists do not pay for with the variance branch (general kernel
+        // us, then its multiple by lanes: 125 tiles 4 pairs 5.2, 1.70, 41 pairs 9.9, 1.03, 207 pairs 30, 0.81; 1,728 tiles
+        // 3.7 pairs 18, 1.56, 8.3 19, 1.47, 10.7 30, 0.97, 21 46, 0.74; 4,096 tiles 2.4 pairs 36, 1.40, 12 61, 0.95;
+        // 13,824 tiles 1.4 pairs 112, 1.15, 2.8 142, 1.04, 7.0 179, 0.89).
+        const bool short_lists = kVar && pairs < 4000 + 10 * (n_tiles < 4096 ? n_tiles : 4096);
+        if (g.T == 8 && !short_lists) {
             const unsigned grid = g.tiles_x * g.tiles_y * g.tiles_z;
             voxel_bwd_lanes_kernel<kVar, kBulk><<<grid, kVoxLaneThreads, 0, stream>>>(
                 rec, chain_var, offsets, ids, g, v_vol, v_vol_var, grads, sl);
@@ -2311,9 +2319,6 @@ int launch_vbwd_p(const VoxelGeom& g, const Rec3D<S>* rec, bool chain_var, const
         }
     }
     if constexpr (std::is_same<S, float>::value && kBeta) {
-        // With the count on the device, the slots' capacity stands for it.
-        const uint64_t n_tiles = uint64_t(g.tiles_x) * g.tiles_y * g.tiles_z;
-        const uint64_t pairs = g.n_dev == nullptr ? g.n_isects : sl.slots != nullptr ? sl.capacity : 0u;
         const uint32_t shares = g.T == 8 ? beta_bwd_shares(n_tiles, pairs, g.N) : 0u;
         if (shares != 0u) {
             voxel_beta_bwd_kernel<kVar, kBulk>
