@@ -1554,7 +1554,9 @@ int launch_record_bwd_t(const RasterGeom& g, const Rec2D<S>* rec, const ushort4*
     // 1.133 ms with two, 1.141 with one); at 2.6 waves two batches leave a short last wave (0.227 / 0.205 ms).
     const size_t wave = size_t(sms > 0 ? sms : 148) * size_t(per_sm > 0 ? per_sm : 1);
     const size_t runs = (total + kRecBwdThreads - 1) / kRecBwdThreads;
-    const size_t batches = runs >= 64 * wave ? 4 : runs >= 4 * wave ? 2 : 1;
+    // In fp64 a batch lasts long enough for the dispatch not to matter, and a short last wave does: one up to 64 waves
+    // (50,000 primitives, 17 views of 333 x 517: 2.09 ms the VJP call with two, 2.03 with one).
+    const size_t batches = runs >= 64 * wave ? 4 : runs >= 4 * wave && sizeof(S) == 4 ? 2 : 1;
     const size_t blocks = (runs + batches - 1) / batches;
     raster_record_bwd_kernel<S, kBeta, kVar, kAbs><<<unsigned(blocks), kRecBwdThreads, 0, stream>>>(
         rec, rects, var_q, g.C, g.N, g.width, g.height, g.T, v_render, v_render_var, grads, v_abs, v_unc,
