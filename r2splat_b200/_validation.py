@@ -9,8 +9,8 @@ callers and tests match on them.
 The reference evaluates each value check (finiteness, ranges, camera
 structure) with its own device reduction and host read. Here, inside
 ``deferred_value_checks()``, value checks are queued in the order they are
-made and evaluated together by one kernel (``r2s_check_values``) and one host
-read, when the block ends or when a host-side check raises; the first failing
+made and evaluated together by one kernel (``r2s_check_values_host``) and one host
+wait, when the block ends or when a host-side check raises; the first failing
 check in call order raises, so the error a caller sees is the reference's.
 """
 

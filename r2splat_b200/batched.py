@@ -427,7 +427,7 @@ class Autotuner:
         for tile in self.TILES:
             for batch in self.BATCHES:
                 if tile == 8 and batch > 64:
-                    continue  # an 8x8 tile has 64 pixels: the staging batch is capped at the thread count
+                    continue  # the forward stages at most 64 records a batch at tile 8 (224 at tile 16)
                 scene = make_scene(tile, batch)
                 scene.step()
                 torch.cuda.synchronize()

@@ -3,31 +3,30 @@
 // records.
 //
 // Layout and schedule (B200):
-//  * one CTA per (tile, camera); blockIdx.x = tile, blockIdx.y = camera, so
-//    CTAs run camera-major and one camera's records ([N] x 32 B) stay resident
-//    in L2 while its tiles are processed;
-//  * the tile's intersection list (contiguous in the sorted flatten_ids) is
-//    staged in shared memory in batches, each thread gathering one 32-byte
-//    record with two 16-byte cp.async copies, double-buffered so the next
-//    batch's gather overlaps the current batch's arithmetic;
-//  * each staged record gets a conservative pixel box on this tile (the
-//    pixels where its sample can pass the contribution test), computed once
-//    per CTA by the thread that staged it;
-//  * forward: one pixel per thread, each warp owning an 8x4 block of the
-//    tile; a warp ballots which staged records' boxes meet its block and
-//    evaluates only those, in list order, so every pixel still sums its
-//    contributions in the reference's order;
-//  * backward: one warp per record, evaluating only the pixels of its box
-//    (about a third of the tile for CT-sized Gaussians), accumulating six to
-//    eight partial sums per lane, reducing them with a recursive-halving warp
-//    sum and adding them to the packed adjoints with vector atomics.
+//  * forward: one CTA per (tile, camera). The tile's intersection list
+//    (contiguous in the sorted flatten_ids) is staged in shared memory in
+//    batches, each thread gathering one 32-byte record with two 16-byte cp.async
+//    copies, triple-buffered so the next batch's gather overlaps the current
+//    one's arithmetic. The thread that staged a record gives it a conservative
+//    pixel box on the tile (raster_box.cuh), and only the pixel blocks that the
+//    box meets evaluate it, in list order, so every pixel sums its contributions
+//    in the reference's order. Three kernels: raster_fwd_group_kernel (fp32,
+//    tiles 8, 16 and 32: a hit list per 4x4 or 8x8 block, tile rows of all
+//    cameras from the middle outwards), raster_fwd_pair_kernel (fp32, short
+//    lists and other tiles: two pixels per lane, warps of 8x8 pixels, camera by
+//    camera) and raster_fwd_kernel (fp64: warps of 8x4 pixels);
+//  * backward: raster_record_bwd_kernel, by records: groups of 8, 16 or 32 lanes
+//    walk the pixels of a record's box over the whole image and write its packed
+//    adjoints once, without atomics. fp32 Gaussians with the variance branch can
+//    run tile-parallel instead (raster_tile_bwd.cu). raster_bwd_kernel, by tiles
+//    with vector atomics into the packed adjoints, serves the low-level calls.
 //
 // Per-sample arithmetic keeps the reference's expression forms
 // (RasterizeToPixelsFwd.cu:160-177, :664-680; RasterizeToPixelsBwd.cu:417-468,
 // :910-945): the contribution thresholds (|alpha| < 1e-5, sigma < 0, d2 >= 1)
 // decide which samples count, so alpha must round exactly as the reference's
-// does. Each thread evaluates one pixel per record, as in the reference's
-// one-pixel-per-thread loops, so the compiler contracts the same multiply-adds.
+// does. Where a lane evaluates several pixels the contraction that nvcc gives the
+// reference's one-pixel-per-thread loops is spelled out.
 #include <type_traits>
 
 #include "common.cuh"
