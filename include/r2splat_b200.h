@@ -360,8 +360,8 @@ int r2s_raster_project(int dtype, const void* means, const void* covars, const v
 int r2s_scan_tile_counts(const int32_t* counts, uint64_t n, int64_t* cum, void* workspace,
                          size_t workspace_bytes, void* stream);
 
-/* *out (device) = the number of nonzero counts [n]: the records that meet any tile. */
-int r2s_count_nonzero(const int32_t* counts, uint64_t n, int64_t* out, void* stream);
+/* *out (device) = the number of nonempty rectangles among rects [n,4]: the records that meet any tile. */
+int r2s_raster_count_visible(const uint16_t* rects, uint64_t n, int64_t* out, void* stream);
 
 /* Emits the sorted 2D intersections from precomputed rectangles (no radii).
  * n_isects: the scan's last entry, which every array is sized by; nothing is

@@ -90,12 +90,11 @@ def _read_total(cum: Tensor, before=None) -> int:
     return ctypes.c_int64.from_address(_ptr(host)).value
 
 
-def _read_sizes(cum: Tensor, counts: Tensor, before=None) -> tuple[int, int]:
-    """(intersections, records that have any) of a scan and its counts; both copies are enqueued before either wait."""
-    nonzero = torch.empty(1, dtype=torch.int64, device=counts.device)
-    _backend.call("r2s_count_nonzero", _ptr(counts), counts.numel(), _ptr(nonzero), _stream(counts.device))
-    visible = []
-    return _read_total(cum, lambda: visible.append(_read_total(nonzero, before))), visible[0]
+def _read_visible(rects: Tensor) -> int:
+    """The number of records with a tile rectangle. Waits for the work queued before it."""
+    visible = torch.empty(1, dtype=torch.int64, device=rects.device)
+    _backend.call("r2s_raster_count_visible", _ptr(rects), rects.numel() // 4, _ptr(visible), _stream(rects.device))
+    return _read_total(visible)
 
 
 def beta_path_ratio(beta: Tensor) -> Tensor:
@@ -198,20 +197,19 @@ class VoxelState:
 
 
 def raster_intersections(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps, radius_clip,
-                         tile_size=RASTER_TILE, before_count=None, count_visible=False):
+                         tile_size=RASTER_TILE, before_count=None):
     """Projection + packing + sorted tile intersections.
 
-    Returns (records, offsets, isect_ids, flatten_ids, M, rects, cum, visible); rects [C,N,4] are the tile rectangles,
-    cum the inclusive scan of the per-record tile counts, which the VJP's slots are numbered by, and visible the number
-    of records with tiles (None unless ``count_visible``).
+    Returns (records, offsets, isect_ids, flatten_ids, M, rects, cum); rects [C,N,4] are the tile rectangles and
+    cum the inclusive scan of the per-record tile counts, which the VJP's slots are numbered by.
     ``before_count`` runs just before the host reads the intersection count (the pending input checks).
     """
     records, rects, counts = _raster_project(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps,
                                              radius_clip, tile_size)
     cum = _raster_scan(counts)
-    m, visible = _read_sizes(cum, counts, before_count) if count_visible else (_read_total(cum, before_count), None)
+    m = _read_total(cum, before_count)
     isect_ids, flatten_ids, offsets = _raster_lists(rects, cum, m, width, height, tile_size)
-    return records, offsets, isect_ids, flatten_ids, m, rects, cum, visible
+    return records, offsets, isect_ids, flatten_ids, m, rects, cum
 
 
 def _raster_project(means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps, radius_clip, tile_size):
@@ -263,7 +261,7 @@ def raster_vjp_has_tile_form(dtype, beta: bool, variance: bool, tile_size, width
             and max(width, height) < 65536)
 
 
-def raster_vjp_takes_tiles(n_isects, n_visible, n_lists) -> bool:
+def raster_vjp_takes_tiles(n_isects, n_records, n_lists, count_visible) -> bool:
     """Whether a VJP that has the tile form takes it: by its intersections, the records that have any, and the lists.
 
     The tile walk evaluates whole 8x8 blocks at 0.11 ns a pair, the record walk the pixels of each record's box at some
@@ -272,12 +270,20 @@ def raster_vjp_takes_tiles(n_isects, n_visible, n_lists) -> bool:
     984 / 537, 7.8 511 / 286, 29 1132 / 361). A list costs 2.1 ns by itself, its tile's adjoints being staged however
     short it is: 65,536 lists of 4, 9 and 18 records of 3.7 tiles take 164, 207 and 271 us against 81, 163 and 277 by
     records. Up to 4,096 lists that is below the record walk's own latency (1,000 records on 1,024 lists: 63 / 19).
-    The rule depends on the scene alone, not on whether the lists are still held, so a rebuilt backward gives the same
-    gradients.
+
+    Both conditions grow with the tiles a visible record meets. If they hold with all records counted as visible, they
+    hold; if not, ``count_visible`` is asked, for which the host waits (detectors that show a part of the scene: 71 x 521,
+    94 views, 1.6 tiles a record and 3.7 a visible one, 1858 / 978 us). Up to 65,536 records, which either form walks in
+    20 to 60 us, all are taken as visible. The rule depends on the scene alone, not on whether the lists are still held,
+    so a rebuilt backward gives the same gradients.
     """
-    return (4 * n_isects >= 9 * n_visible
-            and n_isects * (2 * n_isects - 3 * n_visible) >= 56 * n_visible * max(n_lists - 4096, 0)
-            and n_isects * RASTER_SLOT_BYTES <= RASTER_SLOT_BUDGET_BYTES)
+    def pays(visible):
+        return (4 * n_isects >= 9 * visible
+                and n_isects * (2 * n_isects - 3 * visible) >= 56 * visible * max(n_lists - 4096, 0))
+
+    if n_isects * RASTER_SLOT_BYTES > RASTER_SLOT_BUDGET_BYTES:
+        return False
+    return pays(n_records) or (n_records > 65_536 and pays(count_visible()))
 
 
 IMAGE_LOSS_KINDS = {"mse": 0, "l1": 1}  # R2S_IMAGE_LOSS_MSE, R2S_IMAGE_LOSS_L1
@@ -316,11 +322,9 @@ def raster_forward(means, quats, scales, densities, viewmats, Ks, width, height,
     c = viewmats.shape[0]
     covars = _covariances(quats, scales)
     ratio = beta_path_ratio(beta) if beta is not None else None
-    has_tile_vjp = raster_vjp_has_tile_form(means.dtype, beta is not None, uncertainty is not None, tile_size, width,
-                                            height)
-    records, offsets, isect_ids, flatten_ids, m, rects, cum, visible = raster_intersections(
+    records, offsets, isect_ids, flatten_ids, m, rects, cum = raster_intersections(
         means, covars, densities, beta, ratio, viewmats, Ks, width, height, eps, radius_clip, tile_size,
-        before_count, has_tile_vjp)
+        before_count)
     image = means.new_empty((c, height, width))
     variance = torch.empty_like(image) if uncertainty is not None else None
     tx = (width + tile_size - 1) // tile_size
@@ -339,8 +343,8 @@ def raster_forward(means, quats, scales, densities, viewmats, Ks, width, height,
     state = RasterState(covars, records, offsets, isect_ids, flatten_ids, ratio, m, width, height, tile_size,
                         extra={"rects": rects})
     # The scan (8 bytes a record: 512 MB at 500,000 primitives and 128 views) is kept only for the VJP that reads it.
-    if has_tile_vjp:
-        state.extra.update(cum=cum, visible=visible)
+    if raster_vjp_has_tile_form(means.dtype, beta is not None, uncertainty is not None, tile_size, width, height):
+        state.extra["cum"] = cum
     output = image if uncertainty is None else (image, variance)
     if image_loss is None:
         return output, state
@@ -390,14 +394,14 @@ def _raster_vjp_lists(state: RasterState, dtype, beta: bool, variance: bool):
     try:
         held = state.offsets is not None and "cum" in state.extra
         if held:
-            cum, m, visible = state.extra["cum"], state.n_isects, state.extra["visible"]
+            cum, m = state.extra["cum"], state.n_isects
         else:
             # Rectangles are in tiles, below 2^13 on this path, so 16-bit differences are exact.
             x0, y0, x1, y1 = rects.unbind(-1)
             counts = ((x1 - x0).int() * (y1 - y0)).contiguous()
             cum = _raster_scan(counts)
-            m, visible = _read_sizes(cum, counts)
-        if not raster_vjp_takes_tiles(m, visible, n_lists):
+            m = _read_total(cum)
+        if not raster_vjp_takes_tiles(m, rects.shape[0] * rects.shape[1], n_lists, lambda: _read_visible(rects)):
             return None
         if held:
             flatten_ids, offsets = state.flatten_ids, state.offsets

@@ -514,12 +514,15 @@ __device__ __forceinline__ void block_scatter_ballot(const uint32_t* __restrict_
     }
 }
 
-// The number of nonzero counts, added up block by block (whole numbers: any order gives the same sum).
-__global__ void __launch_bounds__(256) count_nonzero_kernel(const int32_t* __restrict__ counts, uint64_t n,
+// The number of records with a tile rectangle, added up block by block (whole numbers: any order gives the same sum).
+__global__ void __launch_bounds__(256) count_visible_kernel(const ushort4* __restrict__ rects, uint64_t n,
                                                             unsigned long long* __restrict__ out) {
     uint32_t mine = 0u;
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) mine += counts[i] != 0;
+    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const ushort4 r = rects[i];
+        mine += r.z > r.x && r.w > r.y;
+    }
     mine = __reduce_add_sync(0xffffffffu, mine);
     __shared__ uint32_t s_sum[8];
     if ((threadIdx.x & 31u) == 0u) s_sum[threadIdx.x >> 5] = mine;
@@ -868,15 +871,15 @@ int r2s_scan_tile_counts(const int32_t* counts, uint64_t n, int64_t* cum, void* 
                                                as_stream(stream));
 }
 
-int r2s_count_nonzero(const int32_t* counts, uint64_t n, int64_t* out, void* stream) {
-    R2S_REQUIRE(out != nullptr && (counts != nullptr || n == 0), R2S_ERR_ARGUMENT, "counts and out must be non-null");
+int r2s_raster_count_visible(const uint16_t* rects, uint64_t n, int64_t* out, void* stream) {
+    R2S_REQUIRE(out != nullptr && (rects != nullptr || n == 0), R2S_ERR_ARGUMENT, "rects and out must be non-null");
     cudaStream_t st = as_stream(stream);
     if (cudaMemsetAsync(out, 0, sizeof(int64_t), st) != cudaSuccess) return fail(R2S_ERR_CUDA, "memset failed");
     if (n == 0) return R2S_OK;
-    const uint64_t blocks = (n + 2047) / 2048;  // eight counts a thread, up to eight blocks a SM
-    count_nonzero_kernel<<<unsigned(blocks < 1184 ? blocks : 1184), 256, 0, st>>>(
-        counts, n, reinterpret_cast<unsigned long long*>(out));
-    return check_launch("count_nonzero");
+    const uint64_t blocks = (n + 2047) / 2048;  // eight rectangles a thread, up to eight blocks a SM
+    count_visible_kernel<<<unsigned(blocks < 1184 ? blocks : 1184), 256, 0, st>>>(
+        reinterpret_cast<const ushort4*>(rects), n, reinterpret_cast<unsigned long long*>(out));
+    return check_launch("count_visible");
 }
 
 size_t r2s_isect_emit_workspace(uint64_t n_isects, uint64_t n_keys) {

@@ -79,7 +79,7 @@ SIGNATURES: dict[str, tuple] = {
     "r2s_beta_path_factor": (I32, [I32, P, U32, P, P, P]),
     "r2s_raster_project": (I32, [I32, P, P, P, P, P, P, P, U32, U32, U32, U32, F32, F64, F32, U32, U32, U32,
                                  P, P, P, P]),
-    "r2s_count_nonzero": (I32, [P, U64, P, P]),
+    "r2s_raster_count_visible": (I32, [P, U64, P, P]),
     "r2s_raster_emit": (I32, [P, U32, U32, U32, U32, P, I64, P, P, P, P, SZ, P]),
     "r2s_raster_render": (I32, [I32, P, P, I32, P, P, U32, U32, U32, U32, U32, U32, U32, U32, P, P, P]),
     "r2s_raster_render_bwd": (I32, [I32, P, P, I32, I32, P, P, P, P, U32, U32, U32, U32, U32, U32, U32, U32,

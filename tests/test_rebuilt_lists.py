@@ -32,7 +32,7 @@ def test_the_lists_are_sized_by_the_rectangles_own_count(monkeypatch):
     monkeypatch.setattr(_fused._backend, "library", lambda: type("L", (), {
         "r2s_isect_emit_workspace": staticmethod(lambda m, keys: m)})())
     monkeypatch.setattr(_fused, "_raster_scan", lambda c: c.flatten().to(torch.int64).cumsum(0))
-    monkeypatch.setattr(_fused, "_read_sizes", lambda cum, counts: (int(cum[-1]), int((counts != 0).sum())))
+    monkeypatch.setattr(_fused, "_read_total", lambda cum: int(cum[-1]))
     monkeypatch.setattr(torch.cuda.nvtx, "range_push", lambda name: None)
     monkeypatch.setattr(torch.cuda.nvtx, "range_pop", lambda: None)
     for stale in (None, 3, 10_000):
@@ -186,11 +186,26 @@ def test_without_room_for_slots_or_lists_the_records_are_walked(device, monkeypa
 
 
 def test_rule_for_the_tile_walk():
-    takes = _fused.raster_vjp_takes_tiles
+    def takes(isects, records, lists, visible=None):
+        asked = []
+
+        def count():
+            asked.append(True)
+            return visible
+
+        taken = _fused.raster_vjp_takes_tiles(isects, records, lists, count)
+        assert bool(asked) == (visible is not None)  # counted only where it can change the answer
+        return taken
+
     assert takes(0, 0, 10**6)  # nothing to walk
     assert takes(9, 4, 4096) and not takes(8, 4, 4096)  # 2.25 tiles a record
+    assert not takes(65_536, 65_536, 100)
+    assert takes(225_000, 200_000, 100, visible=100_000) and not takes(225_000, 200_000, 100, visible=100_001)
     # 65,536 lists of 3.7 tiles a record: 18 records a list pay for the lists, nine do not.
-    assert takes(65536 * 18, 65536 * 18 * 10 // 37, 65536) and not takes(65536 * 9, 65536 * 9 * 10 // 37, 65536)
+    for records, pays in ((18, True), (9, False)):
+        n = 65536 * records
+        assert takes(n, n * 10 // 37, 65536, visible=None if pays else n * 10 // 37) == pays
+        assert takes(n, n, 65536, visible=n * 10 // 37) == pays
     budget = _fused.RASTER_SLOT_BUDGET_BYTES // _fused.RASTER_SLOT_BYTES
     assert takes(budget, 1000, 1) and not takes(budget + 1, 1000, 1)
 
@@ -198,10 +213,35 @@ def test_rule_for_the_tile_walk():
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [0, 1, 255, 2049, 3_000_001])
 def test_records_with_tiles_are_counted(device, n):
-    counts = torch.randint(-1, 3, (n,), generator=torch.Generator().manual_seed(n)).to(device, torch.int32)
-    out = torch.full((1,), 99, dtype=torch.int64, device=device)
-    _backend.call("r2s_count_nonzero", _ptr(counts), n, _ptr(out), _fused._stream(device))
-    assert int(out) == int((counts != 0).sum())
+    rects = torch.randint(0, 3, (n, 4), generator=torch.Generator().manual_seed(n)).to(device, torch.int16)
+    x0, y0, x1, y1 = rects.unbind(-1)
+    assert _fused._read_visible(rects) == int(((x1 > x0) & (y1 > y0)).sum())
+
+
+@pytest.mark.gpu
+def test_partly_visible_scene_counts_and_takes_tiles(device, monkeypatch):
+    """More than 65,536 records, most of them off the detectors: fewer than 2.25 tiles a record, more a visible one."""
+    n, size = 30_000, (24, 640)
+    means, quats, scales, dens, _, q = (None if t is None else t.to(device) for t in
+                                        scenes.random_primitives(n, 9, 0.02, 0.3, uncertainty_max=0.1))
+    viewmats, Ks = (t.to(device) for t in scenes.orbit_cameras(3, 3.0, 700.0, size[1], size[0]))
+    v = torch.randn((3,) + size, device=device, generator=torch.Generator(device=device).manual_seed(1))
+    decisions, rule = [], _fused.raster_vjp_takes_tiles
+
+    def watched(isects, records, lists, count):
+        decisions.append((isects, records, rule(isects, records, lists, count)))
+        return decisions[-1][2]
+
+    monkeypatch.setattr(_fused, "raster_vjp_takes_tiles", watched)
+    grads = []
+    for release in (False, True):
+        _, ctx = r2s.rasterize_fwd(means, quats, scales, dens, viewmats, Ks, size, uncertainty=q)
+        if release:
+            explicit.release_intersection_lists(ctx)
+        grads.append(r2s.rasterize_bwd(ctx, v, v))
+    assert len(decisions) == 2 and all(4 * m < 9 * c and c > 65_536 and taken for m, c, taken in decisions)
+    for name in FIELDS:
+        assert torch.equal(getattr(grads[0], name), getattr(grads[1], name))
 
 
 @pytest.mark.gpu
