@@ -85,6 +85,11 @@ ACCUMULATE_KERNELS = {
     "voxel_render_bwd": ("voxel_bwd_lanes_kernel (one lane per (tile, primitive) pair walking the 8^3 tile in "
                          "lockstep)"),
 }
+# The kernels of Beta workloads where they are others.
+BETA_ACCUMULATE_KERNELS = {
+    "voxel_render": "voxel_beta_fwd_kernel (tile forward, a warp walks the records' boxes)",
+    "voxel_render_bwd": "voxel_beta_bwd_kernel (eight lanes per (tile, primitive) pair on its box's rows)",
+}
 # FP32 operations per sample of the Beta raster VJP with the variance branch in the reference's form
 # (RasterizeToPixelsBwd.cu:817-1046), counted by the same rule: offsets 2, d^2 9, h 1, pow argument 1,
 # alpha 1, variance terms 7, w with h^(beta - 1) 6, w dx and w dy 2, their moments 8, g vis 2,
@@ -105,10 +110,9 @@ WORKLOAD_TEXT = {
              "volume 384^3, adjoints v ~ N(0, 1) and v_var ~ N(0, 0.1), variance branch attached"),
 }
 # DRAM bytes (read + write) of one record-parallel raster VJP launch, from ncu
-# (dram__bytes_read.sum + dram__bytes_write.sum, one pass, one full-size launch of the
-# shipped kernel, profiles/ct_fit_step_launch_list.md): 552.60 MB read, 372.58 MB written
-# at the CT workload.
-RASTER_VJP_TRAFFIC_BYTES = {"ct": 552.60e6 + 372.58e6}
+# (dram__bytes_read.sum + dram__bytes_write.sum, one pass, one full-size launch,
+# profiles/accumulate_kernels_ncu.md): 533.91 MB read, 368.28 MB written at the CT workload.
+RASTER_VJP_TRAFFIC_BYTES = {"ct": 533.91e6 + 368.28e6}
 
 
 # --------------------------------------------------------------------------- utilities
@@ -1058,7 +1062,7 @@ def accumulate_rooflines(workload, stages, steps, raster_evals, voxel_evals, fp3
             continue
         ms = stages[stage] / steps
         evals = raster_evals if stage.startswith("raster") else voxel_evals
-        entry = {"kernel": kernel, "ms": ms, "samples": evals}
+        entry = {"kernel": BETA_ACCUMULATE_KERNELS.get(stage, kernel) if beta else kernel, "ms": ms, "samples": evals}
         if beta:
             if stage == "raster_render_bwd":
                 entry["ops_per_sample"] = BETA_VAR_VJP_FLOPS_PER_EVAL

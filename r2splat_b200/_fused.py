@@ -266,14 +266,15 @@ def raster_vjp_takes_tiles(n_isects, n_records, n_lists, count_visible) -> bool:
 
     The tile walk evaluates whole 8x8 blocks at 0.11 ns a pair, the record walk the pixels of each record's box at some
     0.075 ns a pair for each tile that the record meets, so tiles pay once a record meets 2.25 of them on average
-    (us by records / by tiles: 2.08 tiles a record 102 / 120, 2.21 202 / 226, 2.35 1564 / 1329, 2.9 1489 / 1186, 4.4
-    984 / 537, 7.8 511 / 286, 29 1132 / 361). A list costs 2.1 ns by itself, its tile's adjoints being staged however
-    short it is: 65,536 lists of 4, 9 and 18 records of 3.7 tiles take 164, 207 and 271 us against 81, 163 and 277 by
-    records. Up to 4,096 lists that is below the record walk's own latency (1,000 records on 1,024 lists: 63 / 19).
+    (us by records / by tiles: 1.7 tiles a record 115 / 160, 2.08 217 / 249, 2.21 211 / 226, 2.35 1573 / 1331, 2.9
+    1518 / 1190, 4.4 1038 / 538, 7.8 566 / 287, 29 2901 / 806). A list costs 2.1 ns by itself, its tile's adjoints being
+    staged however short it is: 65,536 lists of 4, 9 and 18 records of 3.7 tiles take 162, 208 and 272 us against 113,
+    199 and 305 by records. Up to 4,096 lists that is below the record walk's own latency (1,000 records on 1,024 lists:
+    91 / 19).
 
     Both conditions grow with the tiles a visible record meets. If they hold with all records counted as visible, they
     hold; if not, ``count_visible`` is asked, for which the host waits (detectors that show a part of the scene: 71 x 521,
-    94 views, 1.6 tiles a record and 3.7 a visible one, 1858 / 978 us). Up to 65,536 records, which either form walks in
+    94 views, 1.6 tiles a record and 3.7 a visible one, 1893 / 979 us). Up to 65,536 records, which either form walks in
     20 to 60 us, all are taken as visible. The rule depends on the scene alone, not on whether the lists are still held,
     so a rebuilt backward gives the same gradients.
     """

@@ -437,10 +437,10 @@ __global__ void __launch_bounds__(kMaxThreads) raster_fwd_pair_kernel(
 // first and the last CTAs are short (with 8x8 blocks at 64 views: 3.86 ms
 // camera by camera, 3.58 ms this way).
 //
-// Measured against the pair kernel (B200): the cone-beam scene 4.30 -> 3.49 ms,
-// one view of 100,000 at 512^2 0.119 -> 0.097 ms, 500,000 Beta records with
-// uncertainty, 128 views of 768^2 10.84 -> 8.03 ms. It is bound by instruction
-// issue (86 % of the slots, Beta; special-function unit 57 %).
+// Measured against the pair kernel (B200): the cone-beam scene 4.30 -> 3.10 ms,
+// one view of 100,000 at 512^2 0.121 -> 0.088 ms, 500,000 Beta records with
+// uncertainty, 128 views of 768^2 10.86 -> 7.80 ms. It is bound by instruction
+// issue and the special-function unit (82 and 59 %, Beta; Gaussian 71 and 47 %).
 template <bool kBeta, bool kVar, bool kStrict, int kP>
 __device__ __forceinline__ void group_record(const char* rec, float px, const float2 (&py)[kP], float2 (&acc)[kP],
                                              float2 (&accv)[kP]) {
@@ -1391,9 +1391,10 @@ int launch_fwd_group(const RasterGeom& g, const Rec2D<float>* rec, const float* 
                      const int32_t* ids, float* out, float* out_var, const ImageLossEpilogue<float>& loss,
                      unsigned most, cudaStream_t stream) {
     // At most `most` records a batch: longer batches even out the groups' lists, shorter ones leave room for more
-    // CTAs. Tile 16, ms with 64, 128, 192, 224, 256: 65,536 lists of 720 Gaussians 3.87, 3.52, 3.46, 3.49, 3.54;
-    // 295,000 lists of 480 Beta records 10.0, 8.3, 8.01, 8.03, 8.18; 1024 lists of 360 0.132, 0.105, 0.101, -, 0.095.
-    // Tile 8 (one warp a tile), 8192 lists x 4: 0.628, 0.665, 0.729, 0.812, 0.839.
+    // CTAs. Tile 16, ms with 64, 128, 192, 224, 256: 65,536 lists of 720 Gaussians 3.60, 3.18, 3.09, 3.10, 3.13;
+    // 295,000 lists of 480 Beta records 9.74, 8.08, 7.78, 7.80, 7.93; 1,024 lists of 360 0.121, 0.094, 0.092, 0.089,
+    // 0.086. Tile 8 (one warp a tile): 262,144 lists of 40 0.468, 0.526, 0.689, 0.827, 0.871; 73,728 of 105 Beta records
+    // 0.236, 0.252, 0.324, 0.389, 0.393; 8,192 of 384 0.223, 0.196, 0.198, 0.213, 0.219.
     unsigned batch = g.stage_batch < most ? (g.stage_batch < 1 ? 1u : g.stage_batch) : most;
     batch = (batch + 3u) & ~3u;  // the hit lists are read four entries at a time
     constexpr unsigned groups = (kT / kBlock) * (kT / kBlock), threads = groups * 2u * kBlock;
@@ -1411,8 +1412,8 @@ int launch_fwd_p(const RasterGeom& g, const Rec2D<S>* rec, const S* unc, const i
                  const int32_t* ids, S* out, S* out_var, const ImageLossEpilogue<S>& loss, cudaStream_t stream) {
     if constexpr (std::is_same<S, float>::value) {
         // Tiles of whole 4x4 (8, 16) or 8x8 (32) blocks take the group kernel. Pair kernel against it, ms: 16 views
-        // of 256^2, 40,000 Gaussians 0.246 / 0.138 (tile 8), 0.179 / 0.115 (16), 0.262 / 0.207 (32); 32 views of
-        // 384^2, 100,000 Beta 0.81 / 0.25, 0.364 / 0.240, 0.524 / 0.428. At tile 32 a few lists are better off
+        // of 256^2, 40,000 Gaussians 0.256 / 0.132 (tile 8), 0.177 / 0.119 (16), 0.262 / 0.195 (32); 32 views of
+        // 384^2, 100,000 Beta 0.81 / 0.24, 0.364 / 0.225, 0.526 / 0.407. At tile 32 a few lists are better off
         // with the pair kernel's 16 warps a tile (16 lists of 340: 0.042 / 0.050).
         // Lists of fewer than twelve records on average go to the pair kernel at tile 16: the group kernel's fixed part
         // (three larger buffers, a list per group) is what such a launch costs. 65,536 lists of 1.8, 5.4, 11 and 14

@@ -1527,7 +1527,9 @@ __global__ void __launch_bounds__(kVoxLaneThreads, 4) voxel_bwd_lanes_kernel(
 // to the edge is small, so sums in another order differ by more than rounding
 // usually does.
 // A warp a tile, because tiles hold few Beta pairs (48 in the larger of the
-// scenes below) and a block of eight warps waited on its staging for them.
+// scenes below) and a block of eight warps waited on its staging for them; where
+// tiles are few and lists long, `shares` warps take a part of the list each
+// (beta_bwd_shares).
 // Kernel and slot sum, 100,000 primitives in 192^3: 0.238 -> 0.120 ms; 500,000
 // with the variance in 384^3: 3.07 -> 2.31 ms. 10 blocks a SM (96 registers)
 // against 12 with spills and 8: 2.31 / 2.46 / 2.45 ms. (A lane per voxel of the
